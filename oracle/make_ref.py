@@ -33,10 +33,10 @@ DEFAULT_REFERENCE = Path("/root/reference")
 
 def reference_dir(path=None):
     """The reference checkout: ``path`` if given, else ``$GTRAP_REFERENCE``, else this recipe's
-    default location.  Returns None when the directory does not exist (a GPU host has only the
-    generated source)."""
+    default location.  Returns None when no checkout is there (a GPU host has only the
+    generated source; an empty folder is no checkout)."""
     cand = Path(path or os.environ.get("GTRAP_REFERENCE") or DEFAULT_REFERENCE)
-    return cand if cand.is_dir() else None
+    return cand if (cand / "gtrap").is_dir() else None
 
 
 def _source_module_strings(pyfile: Path):
