@@ -81,6 +81,54 @@ __device__ __forceinline__ uint64_t frac64(float t, float f) {
   return a;
 }
 
+// One step of a compensated sum (Neumaier): v enters unless skip, as selects and no branch, so
+// that a run of steps is one straight chain.
+__device__ __forceinline__ void neumaier_step(float &sum, float &comp, float v, bool skip) {
+  const float t = sum + v;
+  const bool big = fabsf(sum) >= fabsf(v);
+  const float a = big ? sum : v, b = big ? v : sum;
+  const float c = comp + ((a - t) + b);
+  sum = skip ? sum : t;
+  comp = skip ? comp : c;
+}
+
+// The compensated partial p of get_offset's order: the samples p, p + parts, p + 2 parts, ...
+// below n at element stride `stride`, those of negative time left out, in order, kAhead of them
+// loaded before the first is added (the chain waits on its loads, not on the additions).
+template <int kAhead>
+__device__ __forceinline__ double offset_partial(const float *__restrict__ t, const float *__restrict__ x,
+                                                 int64_t p, int64_t parts, int64_t n, int64_t stride) {
+  float sum = 0.0f, comp = 0.0f;
+  const int64_t step = parts * stride;
+  const float *tp = t + p * stride, *xp = x + p * stride;
+  int64_t left = p < n ? (n - 1 - p) / parts + 1 : 0;  // samples of this partial
+  for (; left >= kAhead; left -= kAhead) {
+    float tv[kAhead], xv[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      tv[u] = __ldg(tp);
+      xv[u] = __ldg(xp);
+      tp += step;
+      xp += step;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) neumaier_step(sum, comp, xv[u], tv[u] < 0.0f);
+  }
+  {
+    float tv[kAhead], xv[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      tv[u] = u < left ? __ldg(tp) : -1.0f;
+      xv[u] = u < left ? __ldg(xp) : 0.0f;
+      tp += step;
+      xp += step;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) neumaier_step(sum, comp, xv[u], tv[u] < 0.0f);
+  }
+  return (double)sum + (double)comp;
+}
+
 inline bool is_pow2(uint32_t x) { return x && !(x & (x - 1)); }
 
 inline int ilog2u(uint32_t x) {

@@ -54,3 +54,39 @@ def test_image_offsets_many_curves(cuda):
     got = api.offset(torch.from_numpy(resid).to(cuda), torch.from_numpy(tu).to(cuda)).cpu().numpy()
     ref = oracle.offset(resid, tu)
     np.testing.assert_allclose(got, ref, rtol=2e-6, atol=1e-12)
+
+
+def _offset_in_order(x, t):
+    """One curve's offset in the documented order, float32 Neumaier partials step by step."""
+    n = x.size
+    pad = (-n) % 256
+    v = np.concatenate([x, np.zeros(pad, np.float32)]).reshape(-1, 256)
+    skip = np.concatenate([t < 0, np.ones(pad, bool)]).reshape(-1, 256)
+    s, c = np.zeros(256, np.float32), np.zeros(256, np.float32)
+    for row, no in zip(v, skip):
+        a = np.where(no, 0, row).astype(np.float32)
+        u = s + a
+        e = np.where(np.abs(s) >= np.abs(a), (s - u) + a, (a - u) + s).astype(np.float32)
+        s, c = np.where(no, s, u), np.where(no, c, c + e)
+    part = (s.astype(np.float64) + c.astype(np.float64)).reshape(8, 32)
+    sr = np.zeros(32)
+    for u in range(8):
+        sr = sr + part[u]
+    acc = 0.0
+    for r in range(32):
+        acc += sr[r]
+    return np.float32(acc / n)
+
+
+@pytest.mark.parametrize("nq", [1, 3, 15, 16, 17, 33])
+@pytest.mark.parametrize("n", [1, 256, 4096, 4097, 12289])
+def test_image_offsets_keep_the_order(cuda, n, nq):
+    """The clustered kernel at the edges of its blocks (lanes) and load batches (16 x 256 rows)."""
+    rng = np.random.default_rng(n + nq)
+    resid = rng.normal(1e-3, 1e-3, size=(n, nq)).astype(np.float32)
+    tu = np.tile(np.arange(n, dtype=np.float32)[:, None], (1, nq))
+    tu[rng.random((n, nq)) < 0.1] = -1000.0
+    resid[(tu < 0) & (rng.random((n, nq)) < 0.2)] = np.nan   # masked samples are not looked at
+    got = api.offset(torch.from_numpy(resid).to(cuda), torch.from_numpy(tu).to(cuda)).cpu().numpy()
+    want = np.array([_offset_in_order(resid[:, q], tu[:, q]) for q in range(nq)], np.float32)
+    np.testing.assert_array_equal(got, want)
