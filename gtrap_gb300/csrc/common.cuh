@@ -62,6 +62,14 @@ int ragged_prepare(gtrap_bls_curve *curves, uint32_t ncurves, uint32_t max_n, co
                    const float *x, uint64_t total, void *pool, size_t pool_bytes, uint32_t flags,
                    double xq_cap, cudaStream_t stream);
 
+// Running-median detrend by groups of windows, radii kGroupMinR .. kGroupMaxR: an [n, nq] image,
+// the same one curve (column) a block, and packed curves.
+constexpr uint32_t kGroupMinR = 4, kGroupMaxR = 63;
+int gfilter_groups_image(const float *in, float *out, uint32_t n, uint32_t nq, uint32_t r, cudaStream_t stream);
+int gfilter_groups_columns(const float *in, float *out, uint32_t n, uint32_t nq, uint32_t r, cudaStream_t stream);
+int gfilter_groups_packed(const float *in, float *out, const unsigned long long *off, const uint32_t *n,
+                          uint32_t ncurves, uint32_t max_n, uint32_t r, cudaStream_t stream);
+
 // frac(t*f) * 2^64 for float32 t and f, exact whenever the product is >= 2^-17.
 __device__ __forceinline__ uint64_t frac64(float t, float f) {
   const uint32_t bt = __float_as_uint(t), bf = __float_as_uint(f);

@@ -2,127 +2,43 @@
 //
 // Reference behaviour: gtrap/gfilter.py:13-86 computes, for every sample, the exact
 // (r+1)-th order statistic of the zero-padded window x[i-r .. i+r] by bisection over
-// the window values and writes x[i] - median.  Here every warp owns 32 adjacent curves
-// (one per lane, so each row it touches is one coalesced 128-byte line of the
-// [n, nq] image) and a run of consecutive rows.  Each lane keeps its window sorted in
-// shared memory, laid out [rank][lane] so that every access is bank-conflict free, and
-// slides it one row at a time: the leaving value is located by binary search and the
-// entering value is moved into place by shifting the values between the two.  The
-// median is then the element of rank r.  Work per output is O(displacement) instead
-// of O(window * bisection steps), and the result is the same order statistic, so the
-// residual is bit-identical to the reference's and to scipy.signal.medfilt.
+// the window values and writes x[i] - median.
+//
+// Radii 4 .. 63 (every survey detrend): one thread takes a group of 4, 8 or 16 consecutive rows
+// of a curve and finds their medians in registers (medgroup.cuh).  Image: consecutive threads
+// take consecutive curves of a row group, so a row's loads are coalesced whatever nq.  Packed
+// curves: a block stages its rows in shared memory (padded by one word a group: no conflicts)
+// and writes its residuals back through it.  About 72 min / max instructions a sample at r = 24
+// (issued at half rate) and as many others, whatever the values; before, each lane of a warp slid
+// a sorted window of its own by dependent shared-memory moves.  Before / now, r = 24:
+// 65,536 x 128 479 / 81 us, 65,536 x 8 207 / 16 us, 3001 x 1 98 / 17 us (launch rate), 160 packed
+// curves of 3.5 M samples 462 / 47 us, one of 19,254 69 / 10 us; r = 5 119 / 47, r = 63 2421 / 153
+// us on 65,536 x 128.
+//
+// Other radii: every warp owns 32 adjacent curves (one per lane, so each row it touches is one
+// coalesced 128-byte line of the [n, nq] image) and a run of consecutive rows.  Each lane keeps
+// its window sorted in shared memory, laid out [rank][lane] so that every access is
+// bank-conflict free, and slides it one row at a time: the leaving value is located by binary
+// search and the entering value is moved into place by shifting the values between the two.
+// The median is then the element of rank r.  Work per output is O(displacement) instead of
+// O(window * bisection steps), but each step waits on the one before.
+//
+// Either way the result is the same order statistic, so the residual is bit-identical to the
+// reference's and to scipy.signal.medfilt.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
 
+#include "medwindow.cuh"
+
 namespace {
+
+using gtrap::window_slide;
+using gtrap::window_sort;
 
 __device__ __forceinline__ float load_padded(const float *__restrict__ in, long long i, long long n,
                                              size_t nq, int q, bool qok) {
   return (qok && i >= 0 && i < n) ? __ldg(in + (size_t)i * nq + q) : 0.0f;
-}
-
-// The window S[32 * k], k < w, of one lane (stride 32: [rank][lane]).  Both functions give the
-// element-by-element result of an insertion sort / slide, which keeps equal values in their
-// order.  With `linear` false the window must be sorted (it has never held a NaN): each
-// insertion point is then found by binary search and the elements between move as a block
-// (loads before stores, not one dependent compare per element), which is faster where a lane
-// waits on its own chain (the packed detrend: 5.2 -> 3.3 ms on 2000 uneven curves, a lone
-// 10,069-sample curve 0.112 -> 0.075 ms).  With `linear` true the element-by-element loops
-// run: their cost follows the displacement, which wins where many warps share an SM and the
-// windows are nearly sorted (the image detrend of 128 Kepler-like curves: 0.53 ms against
-// 0.89 ms with binary searches), and they are the order with NaN, which is what it is.
-
-// Moves S[lo..hi) up by one slot (to S[lo+1..hi]).
-__device__ __forceinline__ void window_move_up(float *S, int lo, int hi) {
-  int j = hi;
-  for (; j - 4 >= lo; j -= 4) {
-    const float a0 = S[32 * (j - 1)], a1 = S[32 * (j - 2)], a2 = S[32 * (j - 3)], a3 = S[32 * (j - 4)];
-    S[32 * j] = a0; S[32 * (j - 1)] = a1; S[32 * (j - 2)] = a2; S[32 * (j - 3)] = a3;
-  }
-  for (; j > lo; --j) S[32 * j] = S[32 * (j - 1)];
-}
-
-// Moves S(lo..hi] down by one slot (to S[lo..hi)).
-__device__ __forceinline__ void window_move_down(float *S, int lo, int hi) {
-  int j = lo;
-  for (; j + 4 <= hi; j += 4) {
-    const float a0 = S[32 * (j + 1)], a1 = S[32 * (j + 2)], a2 = S[32 * (j + 3)], a3 = S[32 * (j + 4)];
-    S[32 * j] = a0; S[32 * (j + 1)] = a1; S[32 * (j + 2)] = a2; S[32 * (j + 3)] = a3;
-  }
-  for (; j < hi; ++j) S[32 * j] = S[32 * (j + 1)];
-}
-
-// Sorts the loaded window in place (stable insertion sort).
-__device__ __forceinline__ void window_sort(float *S, int w, bool linear) {
-  for (int k = 1; k < w; ++k) {
-    const float v = S[32 * k];
-    if (!linear) {
-      int lo = 0, hi = k;  // the insertion point: the number of elements <= v
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (S[32 * mid] <= v) lo = mid + 1; else hi = mid;
-      }
-      window_move_up(S, lo, k);
-      S[32 * lo] = v;
-    } else {
-      int j = k;
-      while (j > 0) {
-        const float u = S[32 * (j - 1)];
-        if (u <= v) break;
-        S[32 * j] = u;
-        --j;
-      }
-      S[32 * j] = v;
-    }
-  }
-}
-
-// Slides the window by one row: vold leaves, vnew (!= vold) enters.
-__device__ __forceinline__ void window_slide(float *S, int w, float vold, float vnew, bool linear) {
-  // lowest rank holding the leaving value (present in the window by construction)
-  int lo = 0, hi = w - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (S[32 * mid] < vold) lo = mid + 1; else hi = mid;
-  }
-  int j = lo;
-  if (!linear) {
-    if (vnew > vold) {  // vnew lands before the first element >= vnew above the freed slot
-      int a = j + 1, b = w;
-      while (a < b) {
-        const int mid = (a + b) >> 1;
-        if (S[32 * mid] < vnew) a = mid + 1; else b = mid;
-      }
-      window_move_down(S, j, a - 1);
-      S[32 * (a - 1)] = vnew;
-    } else {            // vnew lands after the last element <= vnew below the freed slot
-      int a = 0, b = j;
-      while (a < b) {
-        const int mid = (a + b) >> 1;
-        if (S[32 * mid] <= vnew) a = mid + 1; else b = mid;
-      }
-      window_move_up(S, a, j);
-      S[32 * a] = vnew;
-    }
-    return;
-  }
-  if (vnew > vold) {
-    while (j + 1 < w) {
-      const float u = S[32 * (j + 1)];
-      if (!(u < vnew)) break;
-      S[32 * j] = u;
-      ++j;
-    }
-  } else {
-    while (j > 0) {
-      const float u = S[32 * (j - 1)];
-      if (!(u > vnew)) break;
-      S[32 * j] = u;
-      --j;
-    }
-  }
-  S[32 * j] = vnew;
 }
 
 __global__ void __launch_bounds__(256) gfilter_kernel(const float *__restrict__ in,
@@ -270,6 +186,7 @@ int gtrap_gfilter(const float *in, float *out, uint32_t n, uint32_t nq, uint32_t
   if (in == out) return fail(GTRAP_ERR_INVALID_ARG, "gfilter: in and out must not alias");
   if (n > 0x7fffffffu || nq > 0x7fffffffu)
     return fail(GTRAP_ERR_INVALID_ARG, "gfilter: n and nq must be below 2^31");
+  if (r >= kGroupMinR && r <= kGroupMaxR) return gfilter_groups_image(in, out, n, nq, r, stream);
   const size_t w = 2 * (size_t)r + 1;
   const size_t per_warp = w * 32 * sizeof(float);
   const size_t budget = (size_t)max_smem_optin();
@@ -306,6 +223,8 @@ int gtrap_gfilter_packed(const float *in, float *out, const uint64_t *off, const
   if (ncurves == 0 || max_n == 0) return GTRAP_OK;
   if (!in || !out || !off || !n) return fail(GTRAP_ERR_INVALID_ARG, "gfilter_packed: null pointer");
   if (in == out) return fail(GTRAP_ERR_INVALID_ARG, "gfilter_packed: in and out must not alias");
+  if (r >= kGroupMinR && r <= kGroupMaxR)
+    return gfilter_groups_packed(in, out, (const unsigned long long *)off, n, ncurves, max_n, r, stream);
   const size_t w = 2 * (size_t)r + 1;
   const size_t per_warp = w * 32 * sizeof(float);
   const size_t budget = (size_t)max_smem_optin();

@@ -1,0 +1,198 @@
+// Running medians of a group of T consecutive windows by one thread, in registers.
+//
+// The windows of T consecutive rows (2r + 1 rows each, r = T A + B with 0 <= B < T) share a core
+// of 2r + 2 - T rows; window k adds the last T - 1 - k of the T - 1 rows before the core (left
+// extras) and the first k of the T - 1 rows behind it (right extras).  As T - 1 rows enter, the
+// median of each window is one of the T middle values of the core (ranks r - T + 1 .. r).
+//   * The core is 2A - 1 whole aligned blocks of T rows and B + 1 rows of the blocks on either
+//     side (padded with -inf on the left and +inf on the right, equally many, which keeps the
+//     middle where it is): each is sorted by a network and they are merged, keeping only the
+//     values that can still be in the middle.
+//   * Then the group is halved: each half's core takes T / 2 more rows (sorted), and the middle
+//     T / 2 of the 3T / 2 values stay, until one value is left for each window: its median.
+// Every step is a compare-exchange of registers, whatever the values: no shared memory, no
+// divergence, no dependence on how far a value travels.  The result is the order statistic
+// itself, so it equals a sorted window's to the bit.  Values must not be NaN (the caller checks).
+#pragma once
+
+namespace gtrap {
+
+__device__ __forceinline__ void cx(float &a, float &b) {
+  const float lo = fminf(a, b), hi = fmaxf(a, b);
+  a = lo;
+  b = hi;
+}
+
+// Batcher's odd-even merge sort of v[0 .. N), N a power of two.
+template <int N>
+__device__ __forceinline__ void net_sort(float (&v)[N]) {
+#pragma unroll
+  for (int p = 1; p < N; p *= 2) {
+#pragma unroll
+    for (int k = p; k >= 1; k /= 2) {
+#pragma unroll
+      for (int j = k % p; j + k < N; j += 2 * k) {
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) cx(v[i + j], v[i + j + k]);
+      }
+    }
+  }
+}
+
+// A bitonic sequence into ascending order.
+template <int N>
+__device__ __forceinline__ void net_clean(float (&v)[N]) {
+#pragma unroll
+  for (int s = N / 2; s >= 1; s /= 2) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (!(i & s)) cx(v[i], v[i + s]);
+  }
+}
+
+// Two ascending sequences of N into one of 2N.
+template <int N>
+__device__ __forceinline__ void net_merge(const float (&a)[N], const float (&b)[N], float (&out)[2 * N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    out[i] = a[i];
+    out[2 * N - 1 - i] = b[i];
+  }
+  net_clean(out);
+}
+
+// The middle H of the 3H values of a (2H, ascending) and b (H, ascending), ascending: the H
+// smallest are among a's lower half and b, the H largest of the rest among what is left of those
+// and a's upper half.
+template <int H>
+__device__ __forceinline__ void net_middle(const float (&a)[2 * H], const float (&b)[H], float (&out)[H]) {
+  float x[H];
+#pragma unroll
+  for (int i = 0; i < H; ++i) x[i] = fmaxf(a[i], b[H - 1 - i]);
+  net_clean(x);
+#pragma unroll
+  for (int i = 0; i < H; ++i) out[i] = fminf(x[i], a[2 * H - 1 - i]);
+  net_clean(out);
+}
+
+// The middle N of two ascending sequences of N, ascending (the N / 2 smallest and the N / 2
+// largest left out).
+template <int N>
+__device__ __forceinline__ void net_middle_of_two(const float (&a)[N], const float (&b)[N], float (&out)[N]) {
+  float lo[N], hi[N];   // the N smallest and the N largest, each bitonic
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    lo[i] = fminf(a[i], b[N - 1 - i]);
+    hi[i] = fmaxf(a[i], b[N - 1 - i]);
+  }
+  float u[N / 2], w[N / 2];   // the upper half of the low ones, the lower half of the high ones
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    u[i] = fmaxf(lo[i], lo[i + N / 2]);
+    w[i] = fminf(hi[i], hi[i + N / 2]);
+  }
+  net_clean(u);
+  net_clean(w);
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    out[i] = u[i];
+    out[i + N / 2] = w[i];
+  }
+}
+
+// The medians of windows K0 .. K0 + T - 1 of a group of T0 from the T middle values of their
+// common core.  left[j] (j = 1 .. T0 - 1): the row that windows 0 .. j - 1 hold; right[j]
+// (j = 0 .. T0 - 2): the row that windows j + 1 .. T0 - 1 hold.
+template <int T0, int T, int K0>
+__device__ __forceinline__ void median_halves(const float (&core)[T], const float (&left)[T0],
+                                              const float (&right)[T0], float (&med)[T0]) {
+  if constexpr (T == 1) {
+    med[K0] = core[0];
+  } else {
+    constexpr int H = T / 2;
+    float e[H], mid[H];
+#pragma unroll
+    for (int i = 0; i < H; ++i) e[i] = left[K0 + H + i];
+    net_sort(e);
+    net_middle<H>(core, e, mid);
+    median_halves<T0, H, K0>(mid, left, right, med);
+#pragma unroll
+    for (int i = 0; i < H; ++i) e[i] = right[K0 + i];
+    net_sort(e);
+    net_middle<H>(core, e, mid);
+    median_halves<T0, H, K0 + H>(mid, left, right, med);
+  }
+}
+
+// Medians of the windows of rows 0 .. T - 1 (relative to the group), r = T A + B.
+// row(k): the value of row k, -r <= k <= T - 1 + r.  `bad` becomes NaN if a value is not finite
+// (its medians are then not to be used).
+template <int T, int A, class Row>
+__device__ __forceinline__ void group_medians(int B, Row row, float (&med)[T], float &bad) {
+  static_assert(A >= 1 && A <= 3, "cores of one to five whole blocks");
+  auto block = [&](int at, float (&v)[T]) {
+#pragma unroll
+    for (int i = 0; i < T; ++i) {
+      v[i] = row(at + i);
+      bad = fmaf(v[i], 0.0f, bad);
+    }
+    net_sort(v);
+  };
+  float core[T];
+  {
+    float edge[2 * T];   // the rows on either side of the whole blocks
+    {
+      float s[T], p[T];
+#pragma unroll
+      for (int i = 0; i < T; ++i) {
+        const bool in = i <= B;
+        s[i] = in ? row(-T * A + T - 1 - i) : -INFINITY;
+        p[i] = in ? row(T * A + i) : INFINITY;
+        bad = fmaf(in ? s[i] : 0.0f, 0.0f, bad);
+        bad = fmaf(in ? p[i] : 0.0f, 0.0f, bad);
+      }
+      net_sort(s);
+      net_sort(p);
+      net_merge(s, p, edge);
+    }
+    float b0[T];
+    if constexpr (A == 1) {
+      block(0, b0);
+      net_middle<T>(edge, b0, core);
+    } else {
+      float pair[2 * T], c[T];
+      block(-T, b0);
+      block(T, c);
+      net_merge(b0, c, pair);
+      if constexpr (A == 2) {   // edge + pair + one block: the middle 2T of the first 4T stay
+        float m[2 * T];
+        net_middle_of_two<2 * T>(edge, pair, m);
+        block(0, b0);
+        net_middle<T>(m, b0, core);
+      } else {                  // edge + two pairs + one block
+        float all[4 * T], m[2 * T];
+        net_merge(edge, pair, all);
+        block(-2 * T, b0);
+        block(2 * T, c);
+        net_merge(b0, c, pair);
+        net_middle<2 * T>(all, pair, m);
+        block(0, b0);
+        net_middle<T>(m, b0, core);
+      }
+    }
+  }
+  float left[T], right[T];
+  const int r = T * A + B;
+  left[0] = right[T - 1] = 0.0f;   // not used
+#pragma unroll
+  for (int j = 1; j < T; ++j) {
+    left[j] = row(j - 1 - r);
+    right[j - 1] = row(r + j);
+    bad = fmaf(left[j], 0.0f, bad);
+    bad = fmaf(right[j - 1], 0.0f, bad);
+  }
+  median_halves<T, T, 0>(core, left, right, med);
+}
+
+}  // namespace gtrap

@@ -132,3 +132,21 @@ def test_gfilter_ties_zeros_and_nan(cuda, kind):
             if clean > 0:
                 np.testing.assert_array_equal(g[:clean], ref[:clean])
                 np.testing.assert_array_equal(img[:clean], ref[:clean])
+
+
+@pytest.mark.parametrize("r", [3, 4, 7, 8, 15, 16, 23, 31, 32, 47, 48, 63, 64])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 130, 2065])
+def test_gfilter_groups_at_their_edges(cuda, n, r):
+    """Every group size and core of the grouped medians, at the ends of its range of radii and
+    just past it, on series shorter and longer than a window, a group and a block, with ties and
+    infinities: image (one, three and 40 curves) and packed, bit-exact against medfilt."""
+    rng = np.random.default_rng(64 * n + r)
+    x = rng.normal(1.0, 1e-3, size=(n, 40)).astype(np.float32)
+    x[:, 1] = rng.integers(0, 3, n)
+    x[rng.random((n, 40)) < 0.002] = np.inf
+    want = oracle.medfilt_residual(x, r)
+    for cols in (slice(0, 1), slice(0, 3), slice(0, 40)):
+        got = api.gfilter(torch.from_numpy(np.ascontiguousarray(x[:, cols])).to(cuda), r).cpu().numpy()
+        np.testing.assert_array_equal(got, want[:, cols])
+    for q, got in enumerate(_packed(cuda, [x[:, q].copy() for q in range(5)] + [x[:n // 2 + 1, 5].copy()], r)[:5]):
+        np.testing.assert_array_equal(got, want[:, q])
