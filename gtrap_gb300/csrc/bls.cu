@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kOffParts) bls_ragged_offset_kernel(gtrap_bls_
   __shared__ double part[kOffParts];
   const gtrap_bls_curve c = curves[blockIdx.x];
   const uint32_t p = threadIdx.x;
-  part[p] = gtrap::offset_partial<16>(t + c.off, resid + c.off, p, kOffParts, c.n, 1);
+  part[p] = gtrap::offset_partial<16>(t + c.off, resid + c.off, p, kOffParts, c.n, 1, true);
   __syncthreads();
   if (p < 32) {
     double sr = 0.0;

@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(256) gfilter_packed_kernel(const float *__rest
 // one partial row + 32u with kOffAhead loads in flight, and block 0 adds the partials out of
 // the cluster's shared memory in the order above.  The form before, one block of 32 lanes a
 // group with eight partials a thread, left most SMs idle and all but nq lanes of a small image.
-// Before / now (n x nq): 65,536 x 128 396 / 46 us, 65,536 x 1 269 / 44 us, 18,000 x 1024
-// 194 / 48 us, 3001 x 1 26.5 / 16.4 us (launches back to back).
+// Before / now (n x nq): 65,536 x 128 396 / 28 us, 65,536 x 1 269 / 22 us, 18,000 x 1024
+// 194 / 45 us, 3001 x 1 26.5 / 17.7 us (launches back to back).
 constexpr int kOffParts = 256;
 constexpr int kOffRanks = kOffParts / 32;
 constexpr int kOffLanes = 16;
@@ -156,8 +156,8 @@ offset_kernel(const float *__restrict__ resid, const float *__restrict__ tu,
   cg::cluster_group cluster = cg::this_cluster();
   const int lane = threadIdx.x, row = threadIdx.y;
   const int q = blockIdx.x * blockDim.x + lane;
-  part[row][lane] = q < nq ? gtrap::offset_partial<kOffAhead>(tu + q, resid + q, row + 32 * (int)blockIdx.y,
-                                                              kOffParts, n, nq) : 0.0;
+  part[row][lane] = gtrap::offset_partial<kOffAhead>(tu + q, resid + q, row + 32 * (int)blockIdx.y, kOffParts, n, nq,
+                                                     q < nq);
   cluster.sync();
   if (blockIdx.y == 0) {  // the cluster's rank 0: the grid has kOffRanks blocks along y
     double sr = 0.0;
