@@ -23,12 +23,12 @@
 //  * prefix: groups of Tg threads turn a histogram into exact integer prefix sums, rounded
 //    to float (correctly below 2^31 in magnitude, within one ulp above), plus the maximum
 //    and minimum of the flux prefix per 32-entry chunk.
-//  * scan: every frequency's running best is seeded from real windows; bound groups of
-//    starts against chunks of ends are dropped when their bound falls below it, rows of the
-//    surviving groups are bounded again, and only rows that pass run a division-free
-//    per-start pre-test and then the exact correctly rounded power with a lowest-(start, end)
-//    tie-break.  Every bound is conservative under float rounding, so the outputs equal an
-//    exhaustive scan of the same prefix arrays.
+//  * scan: every frequency's running best is seeded from real windows; units of 32 starts by 32
+//    ends are dropped when the bound that their chunk statistics give falls below it, the ends
+//    and then the starts of the surviving units are bounded one by one, and only the windows of
+//    ends and starts that pass are compared, by the exact correctly rounded power with a
+//    lowest-(start, end) tie-break.  Every bound is conservative under float rounding, so the
+//    outputs equal an exhaustive scan of the same prefix arrays.
 #include <atomic>
 #include <type_traits>
 
@@ -349,9 +349,6 @@ struct BlsArgs {
   float fmin, df;
 };
 
-// Start bins per scan task (one warp; its lanes take 32 end bins at a time).
-constexpr int kRS = 8;
-
 // Order-preserving key of a window: power (non-negative float bits) in the high word, then
 // the lowest (start, end) -- start < 2^17, end < 2^15 -- as the complement in the low word.
 __device__ __forceinline__ unsigned long long pack_key(float pw, int i, int e) {
@@ -379,6 +376,13 @@ __device__ __forceinline__ float ll2float_fast(long long x) {
 
 constexpr int kSeedStride = 4;  // starts seeded per frequency: every fourth
 
+// The largest value of a warp's lanes (no NaN), in one instruction.
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 __device__ __forceinline__ void group_bar(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -391,22 +395,12 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
   __shared__ unsigned long long best_key[64];    // per frequency: best (power, -start, -end)
   __shared__ unsigned best_thr[64];              // per frequency: running best power (float bits)
   __shared__ unsigned job_next;                  // next scan job to take
-  // fold and prefix scratch, dead once the prefix pass has ended, shares its bytes with the
-  // scan's per-warp start-group statistics (the static total decides whether two blocks of
-  // F = 6 frequencies fit on an SM at nb = 2048)
-  __shared__ union {
-    struct {
-      long long x[kThreads / 32];
-      int c[kThreads / 32];
-      int m[kThreads / 32];                      // per-warp maximum bin count
-      unsigned drop[64];                         // FP32-phase samples landing on bin nb
-    } pre;
-    float2 grp[kThreads / 32][4];                // per warp job: its start groups' flux prefix (min, max)
-  } scr;
-  long long *const scan_x = scr.pre.x;
-  int *const scan_c = scr.pre.c;
-  int *const scan_m = scr.pre.m;
-  unsigned *const drop_cnt = scr.pre.drop;
+  // fold and prefix scratch (the static total decides whether two blocks of F = 6 frequencies
+  // fit on an SM at nb = 2048)
+  __shared__ long long scan_x[kThreads / 32];
+  __shared__ int scan_c[kThreads / 32];
+  __shared__ int scan_m[kThreads / 32];          // per-warp maximum bin count
+  __shared__ unsigned drop_cnt[64];              // FP32-phase samples landing on bin nb
 
   const uint32_t j0 = tj.j0;
   const uint32_t nfrem = tj.nfrem;
@@ -698,75 +692,107 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
     pw = __fdiv_rn(s * s, den);
     return pw > 0.0f;
   };
-  // ---- seed every frequency's running best with real windows: for every fourth start,
-  // widths kma, kma/4 and kma/16 (at least kmi + 1).  Quotients are approximate while
-  // the warp picks its best window; only that window's power is computed exactly and
-  // published, so the seed is the exact power of a real window (a valid lower bound of the
-  // maximum) and may itself be the answer.  Seeding every start instead of every fourth
-  // gives a slightly higher first threshold but costs more than the pruning it adds
-  // (measured: BLS kernel 4 % slower on the uneven mix, 3 % on Kepler-like curves).
+  // ---- seed every frequency's running best with real windows.  A warp takes a frequency and a
+  // part of its starts (the parts fill the block's warps): for every fourth start the widths
+  // kma, kma/4 and kma/16 (at least kmi + 1), then from its best window the best end for that
+  // start and the best start for that end.  Quotients are approximate while the warp picks; only
+  // the last window's power is computed exactly and published, so the seed is the exact power of
+  // a real window (a valid lower bound of the maximum) and may itself be the answer.  The ascent
+  // lifts the seed from 0.74-0.82 to 0.92-0.97 of the maximum (means over curves of 3001 to
+  // 65,536 samples), which halves the units that survive the bounds below.
+  auto approx_power = [&](float2 Pi, float2 Pe) -> float {   // 0 where the window does not count
+    const float s = Pe.x - Pi.x;
+    const float kk = Pe.y - Pi.y;
+    const float den = kk * ((Nf + Pi.y) - Pe.y);
+    const float s2 = s * s;
+    const float q = den > 0.0f ? __fdividef(s2, den) : (den == 0.0f && s2 > 0.0f ? INFINITY : 0.0f);
+    return kk > kkmi_f ? q : 0.0f;
+  };
+  // the value of v on the lane of the largest p > 0 (the lowest such lane); p becomes the largest
+  auto of_best = [&](float &p, int v) -> int {
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(p));
+    const int src = __ffs(__ballot_sync(0xffffffffu, __float_as_uint(p) == m)) - 1;
+    p = __uint_as_float(m);
+    return __shfl_sync(0xffffffffu, v, src);
+  };
   if (kma > kmi) {
-    // each thread takes the starts kSeedStride * (tid + kThreads j) of one frequency at a time
-    // and keeps its best; one warp argmax and one exact quotient per warp and frequency
-    // unrolled by three: independent frequencies' load and shuffle chains interleave
-    // (measured 0.4 % faster than one frequency at a time)
-#pragma unroll 3
-    for (uint32_t f = 0; f < nfrem; ++f) {
+    const int parts = max(1, (kThreads / 32) / (int)nfrem);
+    for (int task = warp; task < (int)nfrem * parts; task += kThreads / 32) {
+      const int f = task % (int)nfrem, part = task / (int)nfrem;
       const float2 *P = reinterpret_cast<const float2 *>(sm + (size_t)f * a.region);
+      const int ns = (nb + kSeedStride - 1) / kSeedStride;   // seeded starts of the frequency
+      const int n0 = ns * part / parts, n1 = ns * (part + 1) / parts;
       float pa = 0.0f;
-      int ib = 0, kb = 0;
-      for (int i = tid * kSeedStride; i < nb; i += kThreads * kSeedStride) {
+      int key = 0;
+      for (int n = n0 + lane; n < n1; n += 32) {
+        const int i = n * kSeedStride;
         const float2 Pi = P[swz(i)];
-        const float Ni = Nf + Pi.y;
 #pragma unroll
         for (int m = 0; m < 6; m += 2) {
           const int k = max(kma >> m, kmi + 1);
-          const float2 Pe = P[swz(i + k)];
-          const float s = Pe.x - Pi.x;
-          const float kk = Pe.y - Pi.y;
-          const float den = kk * (Ni - Pe.y);
-          const float s2 = s * s;
-          const float q = den > 0.0f ? __fdividef(s2, den) : (den == 0.0f && s2 > 0.0f ? INFINITY : 0.0f);
-          if (kk > kkmi_f && q > pa) { pa = q; ib = i; kb = k; }
+          const float q = approx_power(Pi, P[swz(i + k)]);
+          if (q > pa) { pa = q; key = (i << 15) | (i + k); }
         }
       }
-      // warp argmax of the approximate powers (lowest lane on ties)
-      float wp = pa;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) wp = fmaxf(wp, __shfl_xor_sync(0xffffffffu, wp, o));
-      const unsigned who = __ballot_sync(0xffffffffu, pa == wp && wp > 0.0f);
-      if (who && lane == __ffs(who) - 1) {
-        float pw;
-        if (window_power(P, ib, ib + kb, pw)) {
-          atomicMax(best_thr + f, __float_as_uint(pw));
-          atomicMax(best_key + f, pack_key(pw, ib, ib + kb));
+      key = of_best(pa, key);
+      if (pa > 0.0f) {   // uniform
+        int ib = key >> 15, eb = key & 0x7fff;
+        {
+          const float2 Pi = P[swz(ib)];
+          float p = 0.0f;
+          int v = eb;
+          for (int e = ib + kmi + 1 + lane; e <= ib + kma; e += 32) {
+            const float q = approx_power(Pi, P[swz(e)]);
+            if (q > p) { p = q; v = e; }
+          }
+          eb = of_best(p, v);
+        }
+        {
+          const float2 Pe = P[swz(eb)];
+          float p = 0.0f;
+          int v = ib;
+          for (int i = max(0, eb - kma) + lane; i <= min(nb - 1, eb - kmi - 1); i += 32) {
+            const float q = approx_power(P[swz(i)], Pe);
+            if (q > p) { p = q; v = i; }
+          }
+          ib = of_best(p, v);
+        }
+        if (lane == 0) {
+          float pw;
+          if (window_power(P, ib, eb, pw)) {
+            atomicMax(best_thr + f, __float_as_uint(pw));
+            atomicMax(best_key + f, pack_key(pw, ib, eb));
+          }
         }
       }
     }
   }
   __syncthreads();
 
-  // ---- candidate windows [i, e), k = e - i in (kmi, kma], kk > kkmi.  Work unit: a chunk of
-  // 32 consecutive end bins against kGS = 16 consecutive start bins (a bound group).  The power
-  // of every window in the unit is bounded by
+  // ---- candidate windows [i, e), k = e - i in (kmi, kma], kk > kkmi.  Unit: the 32 starts of
+  // one chunk against the 32 ends of another.  The power of every window in the unit is bounded by
   //   max(Pmax - ys_min, ys_max - Pmin)^2 / min(den(kk_lo), den(kk_hi))
-  // (den = kk (N - kk) is concave in kk), and units whose bound is below the frequency's shared
-  // running best (times the pre-test slack) cannot hold the maximum.  A warp job takes four
-  // consecutive bound groups; each lane bounds one (group, chunk) unit.  The warp then takes
-  // the surviving units one at a time, one end bin (row) per lane: each row is bounded the same
-  // way with its own prefix, and rows that pass run the per-start test on the group's two
-  // halves of kRS = 8 starts.  A half is one aligned 8-entry block: its entries are read with
-  // four 16-byte broadcast loads and used in slot order (slot j holds start s0 + (j ^ h),
-  // h = the block's swizzle).  Groups of 16 starts halve the unit bounds of 8-start groups
-  // and leave fewer units to walk; the row bound keeps the halves' tests rare.
-  constexpr int kGS = 2 * kRS;
-  const int ngs_f = (nb + kGS - 1) / kGS;            // bound groups per frequency
-  const int ngrp_f = (ngs_f + 3) / 4;                // warp jobs per frequency
-  const int njob = (kma > kmi) ? (int)nfrem * ngrp_f : 0;
-  const int span_chunks = ((kGS - 1 + kma - kmi - 1) >> 5) + 2;   // chunks one group touches
-  // job / ngrp_f as a multiply-high: exact for job < 2^16 and ngrp_f <= 2^16
-  const unsigned long long jmag = 0xffffffffull / (unsigned)ngrp_f + 1ull;
-  float ys[kRS] = {}, beta[kRS] = {}, gamma[kRS] = {};
+  // (den = kk (N - kk) is concave in kk) from the two chunks' statistics alone, a unit a lane, and
+  // units whose bound is below the frequency's shared running best (times the pre-test slack)
+  // cannot hold the maximum.  The warp then takes the surviving units one at a time: one end a
+  // lane is bounded against the chunk of starts (rows), one start a lane against the rows that
+  // are left (columns), the rows once more against those columns, and the windows of the rows
+  // and columns that are left are compared exactly.  Both sides are narrowed by the same bound, so
+  // of 512 units (nb 2048, kma 205) about 36 survive and four get as far as windows.  Before, units
+  // of 16 starts, one pass over the starts behind the ends, and the unascended seeds: 64 x 4096
+  // samples (nb 1024) 5950 -> 4250 us a call, one curve of 3001 135 -> 105, 160 uneven curves
+  // 12.9 -> 10.8 ms, 8 x 65,536 9.1 -> 8.3 ms.
+  const int nsc = (nb + 31) >> 5;                          // chunks of starts per frequency
+  const int oc0 = (kmi + 1) >> 5;                          // first chunk of ends, from the starts' chunk
+  const int nco = max(1, ((31 + kma) >> 5) - oc0 + 1);     // chunks of ends a chunk of starts reaches
+  const int nunit = nsc * nco;
+  // units a warp job: half a warp's where the tile has few, so that the jobs spread evenly
+  const int upj = (int)nfrem * nunit < 32 * 6 * (kThreads / 32) ? 16 : 32;
+  const int njob_f = (nunit + upj - 1) / upj;
+  const int njob = (kma > kmi) ? (int)nfrem * njob_f : 0;
+  // divisions by njob_f and nco as multiply-highs: exact, dividend times divisor < 2^32
+  const unsigned long long jmag = 0xffffffffull / (unsigned)njob_f + 1ull;
+  const unsigned long long umag = 0xffffffffull / (unsigned)nco + 1ull;
   // Jobs are taken from a shared counter in frequency-major order: a frequency's surviving
   // units cluster in the few jobs whose starts lie near its strongest windows, and a fixed
   // job-to-warp assignment leaves the other warps waiting for those at the block barrier.
@@ -776,217 +802,107 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
     job = __shfl_sync(0xffffffffu, job, 0);
     if (job >= njob) break;
     const int f = (int)(((unsigned long long)(unsigned)job * jmag) >> 32);
-    const int t0 = (job - f * ngrp_f) * 4;           // first bound group of the job
     const float2 *P = reinterpret_cast<const float2 *>(sm + (size_t)f * a.region);
     const float2 *CM = reinterpret_cast<const float2 *>(sm + (size_t)f * a.region + lp);
     const float *CL = reinterpret_cast<const float *>(sm + (size_t)f * a.region + lp + nchunk);
-    for (int cbase = 0; cbase < span_chunks; cbase += 8) {
-      unsigned live;
-      float h_min, h_max;   // flux prefix (min, max) over the lane's half: starts 8 (lane >> 2) ..
-      {
-        // the job's 64 starts, two per lane: per group of 16 the minimum and maximum flux
-        // prefix and the count prefix at its first and last start
-        const int kb = lane >> 3, mb = lane & 7;
-        const int sb = (t0 + kb) * kGS;
-        const int nrs_b = min(kGS, nb - sb);
-        float g_min, g_max, g_c0, g_cl;
-        {
-          const int si = t0 * kGS + 2 * lane;
-          const float2 Pa = si < nb ? P[swz(si)] : make_float2(0.0f, 0.0f);
-          const float2 Pb = si + 1 < nb ? P[swz(si + 1)] : make_float2(0.0f, 0.0f);
-          g_min = fminf(si < nb ? Pa.x : INFINITY, si + 1 < nb ? Pb.x : INFINITY);
-          g_max = fmaxf(si < nb ? Pa.x : -INFINITY, si + 1 < nb ? Pb.x : -INFINITY);
-#pragma unroll
-          for (int o = 1; o < 4; o <<= 1) {
-            g_min = fminf(g_min, __shfl_xor_sync(0xffffffffu, g_min, o));
-            g_max = fmaxf(g_max, __shfl_xor_sync(0xffffffffu, g_max, o));
-          }
-          h_min = g_min;   // the lane's half (8 starts)
-          h_max = g_max;
-          g_min = fminf(g_min, __shfl_xor_sync(0xffffffffu, g_min, 4));
-          g_max = fmaxf(g_max, __shfl_xor_sync(0xffffffffu, g_max, 4));
-          const int r = max(nrs_b, 1) - 1;          // the group's last start, relative
-          g_c0 = __shfl_sync(0xffffffffu, Pa.y, lane & ~7);
-          const float ca = __shfl_sync(0xffffffffu, Pa.y, (lane & ~7) + (r >> 1));
-          const float cb = __shfl_sync(0xffffffffu, Pb.y, (lane & ~7) + (r >> 1));
-          g_cl = (r & 1) ? cb : ca;
-          __syncwarp();  // the previous job's reads of scr.grp are done
-          if (mb == 0) scr.grp[warp][kb] = make_float2(g_min, g_max);
-          __syncwarp();
-        }
-        // bound of unit (group kb, chunk c) on this lane; the count prefix at the last entry of
-        // chunks c - 1 and c widens [kk_lo, kk_hi], which only loosens the bound
-        bool keep = false;
-        if (t0 + kb < ngs_f) {
-          const int b_elo = sb + kmi + 1;
-          const int b_ehi = min(sb + nrs_b - 1 + kma, elast);
-          const int c = (b_elo >> 5) + cbase + mb;
-          if (c <= (b_ehi >> 5)) {
-            const float2 cm = CM[c];
-            const float thr = __uint_as_float(best_thr[f]) * kSlack;
-            const float kk_hi = CL[c] - g_c0;
-            if (kk_hi > kkmi_f) {
-              const float kk_lo = fmaxf((c > 0 ? CL[c - 1] : 0.0f) - g_cl, kkmi_f + 1.0f);
-              const float den_min = fminf(kk_lo * (Nf - kk_lo), kk_hi * (Nf - kk_hi));
-              const float smax = fmaxf(cm.x - g_min, g_max - cm.y);
-              keep = !(den_min > 0.0f && smax * smax < thr * den_min);
-            }
-          }
-        }
-        live = __ballot_sync(0xffffffffu, keep);
+    const int u0 = (job - f * njob_f) * upj;
+    // keep unless the bound of flux span smax over counts in [kk_lo, kk_hi] is below thr
+    auto alive = [&](float smax, float kk_lo, float kk_hi, float thr) -> bool {
+      const float lo = fmaxf(kk_lo, kkmi_f + 1.0f);
+      const float den_min = fminf(lo * (Nf - lo), kk_hi * (Nf - kk_hi));
+      return kk_hi > kkmi_f && !(den_min > 0.0f && smax * smax < thr * den_min);
+    };
+    unsigned live;
+    int us, uc;   // the lane's unit: chunk of starts, chunk of ends
+    {
+      const int u = u0 + lane;
+      us = (int)(((unsigned long long)(unsigned)u * umag) >> 32);
+      uc = us + oc0 + (u - us * nco);
+      bool keep = false;
+      if (lane < upj && u < nunit && 32 * uc <= elast) {
+        const float2 cs = CM[us], ce = CM[uc];
+        // counts at or below the first start and the first end, at the last start and the last end
+        const float s_lo = us > 0 ? CL[us - 1] : 0.0f, e_lo = uc > 0 ? CL[uc - 1] : 0.0f;
+        keep = alive(fmaxf(ce.x - cs.y, cs.x - ce.y), e_lo - CL[us], CL[uc] - s_lo,
+                     __uint_as_float(best_thr[f]) * kSlack);
       }
-      float blo = 0.0f, c0 = 0.0f, bpow = 0.0f;
-      int bk = INT_MAX;  // best window of this lane: (start << 15) | end
-      int s0 = -1;       // first start of the loaded half (-1: none)
-      bool improved = false;
-      // pre-test coefficients of the loaded half at threshold blo, in slot order
-      auto coeffs = [&]() {
-        const float4 *Q = reinterpret_cast<const float4 *>(P + s0);
-#pragma unroll
-        for (int q = 0; q < kRS / 2; ++q) {
-          const float4 v = Q[q];
-          const float a0 = v.y - c0, b0 = (Nf + v.y) - c0;
-          const float a1 = v.w - c0, b1 = (Nf + v.w) - c0;
-          beta[2 * q] = -blo * (a0 + b0);
-          gamma[2 * q] = (blo * a0) * b0;
-          beta[2 * q + 1] = -blo * (a1 + b1);
-          gamma[2 * q + 1] = (blo * a1) * b1;
-        }
-      };
-      // exact evaluation of (slot j, end e): pre-test, then the rounded quotient
-      auto consider = [&](int j, float2 Pe, int e) {
-        const int i = s0 + (j ^ ((s0 >> 4) & 7));
-        const float cr = P[s0 + j].y;
-        const float s = Pe.x - ys[j];
-        const float kk = Pe.y - cr;
-        const float den = kk * ((Nf + cr) - Pe.y);
+      live = __ballot_sync(0xffffffffu, keep);
+    }
+    while (live) {
+      const int src = __ffs(live) - 1;
+      live &= live - 1;
+      const int s32 = 32 * __shfl_sync(0xffffffffu, us, src);
+      const int e32 = 32 * __shfl_sync(0xffffffffu, uc, src);
+      const float thr = __uint_as_float(best_thr[f]) * kSlack;
+      const int e = swz(e32 + lane), i = swz(s32 + lane);   // the lane's end and start
+      const bool e_in = e <= elast && e >= s32 + kmi + 1 && e <= s32 + 31 + kma;
+      const float2 Pe = e_in ? P[e32 + lane] : make_float2(0.0f, 0.0f);
+      const float2 Pi = i < nb ? P[s32 + lane] : make_float2(0.0f, 0.0f);
+      bool row;
+      {
+        const float2 cs = CM[s32 >> 5];
+        const float s_lo = s32 > 0 ? CL[(s32 >> 5) - 1] : 0.0f;
+        row = e_in && alive(fmaxf(Pe.x - cs.y, cs.x - Pe.x), Pe.y - CL[s32 >> 5], Pe.y - s_lo, thr);
+      }
+      unsigned rows = __ballot_sync(0xffffffffu, row);
+      if (!rows) continue;
+      bool col;
+      {
+        const float mx = warp_max(row ? Pe.x : -INFINITY), mn = -warp_max(row ? -Pe.x : -INFINITY);
+        const float c1 = warp_max(row ? Pe.y : -INFINITY), c0 = -warp_max(row ? -Pe.y : -INFINITY);
+        col = i < nb && alive(fmaxf(mx - Pi.x, Pi.x - mn), c0 - Pi.y, c1 - Pi.y, thr);
+      }
+      unsigned cols = __ballot_sync(0xffffffffu, col);
+      if (!cols) continue;
+      {
+        const float mx = warp_max(col ? Pi.x : -INFINITY), mn = -warp_max(col ? -Pi.x : -INFINITY);
+        const float c1 = warp_max(col ? Pi.y : -INFINITY), c0 = -warp_max(col ? -Pi.y : -INFINITY);
+        row = row && alive(fmaxf(Pe.x - mn, mx - Pe.x), Pe.y - c1, Pe.y - c0, thr);
+      }
+      rows = __ballot_sync(0xffffffffu, row);
+      if (!rows) continue;
+      // the windows of these rows and columns, the fewer one at a time against the others' lanes
+      float bpow = 0.0f;
+      int bk = INT_MAX;   // best window of this lane: (start << 15) | end
+      auto consider = [&](float2 A, int ii, float2 B, int ee) {
+        const float s = B.x - A.x;
+        const float kk = B.y - A.y;
+        const float den = kk * ((Nf + A.y) - B.y);
         const float s2 = s * s;
         // den <= 0 (a window holding every sample) gives an infinite or negative power
-        if (i < nb && kk > kkmi_f && (den <= 0.0f || fmaf(-blo, den, s2) >= 0.0f)) {
+        if ((unsigned)(ee - ii - kmi - 1) < (unsigned)(kma - kmi) && kk > kkmi_f &&
+            (den <= 0.0f || fmaf(-thr, den, s2) >= 0.0f)) {
           const float pw = __fdiv_rn(s2, den);
-          const int key = (i << 15) | e;
+          const int key = (ii << 15) | ee;
           if (pw > 0.0f && (pw > bpow || (pw == bpow && key < bk))) {
             bpow = pw;
             bk = key;
-            improved = true;
           }
         }
       };
-      auto flush = [&]() {  // warp best of the loaded half into the frequency record
-        if (!__any_sync(0xffffffffu, bk != INT_MAX)) return;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float op = __shfl_down_sync(0xffffffffu, bpow, o);
-          const int ok = __shfl_down_sync(0xffffffffu, bk, o);
-          if (op > bpow || (op == bpow && ok < bk)) { bpow = op; bk = ok; }
-        }
-        if (lane == 0 && bk != INT_MAX) atomicMax(best_key + f, pack_key(bpow, bk >> 15, bk & 0x7fff));
-        bpow = 0.0f;
-        bk = INT_MAX;
-      };
-      while (live) {
-        const int src = __ffs(live) - 1;
-        live &= live - 1;
-        const int k = src >> 3;
-        const int sg = (t0 + k) * kGS;   // first start of the unit's group
-        const int cc = ((sg + kmi + 1) >> 5) + cbase + (src & 7);
-        const int nrs = min(kGS, nb - sg);
-        const int q = 32 * cc + lane;   // physical entry; its logical end bin:
-        const int e = swz(q);
-        const bool row_in = e >= sg + kmi + 1 && e <= min(sg + nrs - 1 + kma, elast);
-        // bound of the lane's row (end e against the group's starts), as the unit bound above
-        // with this end's own prefix: rows that cannot reach the running best skip the
-        // halves' coefficients and per-start tests
-        const float2 Pe = row_in ? P[q] : make_float2(0.0f, 0.0f);
-        bool row = false;
-        {
-          const float kk_hi = Pe.y - P[swz(sg)].y;
-          if (row_in && kk_hi > kkmi_f) {
-            const float2 gx = scr.grp[warp][k];
-            const float thr = __uint_as_float(best_thr[f]) * kSlack;
-            const float kk_lo = fmaxf(Pe.y - P[swz(sg + nrs - 1)].y, kkmi_f + 1.0f);
-            const float den_min = fminf(kk_lo * (Nf - kk_lo), kk_hi * (Nf - kk_hi));
-            const float smax = fmaxf(Pe.x - gx.x, gx.y - Pe.x);
-            row = !(den_min > 0.0f && smax * smax < thr * den_min);
-          }
-        }
-        if (!__any_sync(0xffffffffu, row)) continue;
-        for (int h = 0; h < kGS / kRS; ++h) {
-          const int sh = sg + kRS * h;    // first start of the half
-          if (sh >= nb) break;
-          const int nrs_h = min(kRS, nb - sh);
-          // interior: every (lane, start) of the half has k in range; otherwise windows outside
-          // (kmi, kma] or past the last end are masked before the fast test
-          const bool interior = nrs_h == kRS && 32 * cc >= sh + kRS + kmi && 32 * cc + 31 <= sh + kma;
-          bool go = row && (interior || (e >= sh + kmi + 1 && e <= min(sh + nrs_h - 1 + kma, elast)));
-          // the row bound again over this half's starts alone
-          {
-            const float x_min = __shfl_sync(0xffffffffu, h_min, 8 * k + 4 * h);
-            const float x_max = __shfl_sync(0xffffffffu, h_max, 8 * k + 4 * h);
-            if (go) {
-              const float kk_hi = Pe.y - P[swz(sh)].y;
-              if (kk_hi > kkmi_f) {
-                const float thr = __uint_as_float(best_thr[f]) * kSlack;
-                const float kk_lo = fmaxf(Pe.y - P[swz(sh + nrs_h - 1)].y, kkmi_f + 1.0f);
-                const float den_min = fminf(kk_lo * (Nf - kk_lo), kk_hi * (Nf - kk_hi));
-                const float smax = fmaxf(Pe.x - x_min, x_max - Pe.x);
-                go = !(den_min > 0.0f && smax * smax < thr * den_min);
-              } else {
-                go = false;
-              }
-            }
-          }
-          if (!__any_sync(0xffffffffu, go)) continue;
-          if (sh != s0) {
-            if (s0 >= 0) flush();
-            s0 = sh;
-            const float4 *Q = reinterpret_cast<const float4 *>(P + s0);
-            c0 = P[swz(s0)].y;
-            blo = __uint_as_float(best_thr[f]) * kSlack;
-#pragma unroll
-            for (int w = 0; w < kRS / 2; ++w) {  // entries up to nb + kRS - 1 exist
-              const float4 v = Q[w];
-              ys[2 * w] = v.x;
-              ys[2 * w + 1] = v.z;
-              const float a0 = v.y - c0, b0 = (Nf + v.y) - c0;
-              const float a1 = v.w - c0, b1 = (Nf + v.w) - c0;
-              beta[2 * w] = -blo * (a0 + b0);
-              gamma[2 * w] = (blo * a0) * b0;
-              beta[2 * w + 1] = -blo * (a1 + b1);
-              gamma[2 * w + 1] = (blo * a1) * b1;
-            }
-          } else {
-            const float gb = __uint_as_float(best_thr[f]) * kSlack;
-            if (gb > blo) { blo = gb; coeffs(); }
-          }
-          const int hs = (s0 >> 4) & 7;
-          improved = false;
-          if (go) {
-            const float u = Pe.y - c0;
-            const float G = (blo * u) * u;
-            const unsigned base = (unsigned)(e - s0 - kmi - 1);
-            unsigned neg = 0xffffffffu;
-#pragma unroll
-            for (int j = 0; j < kRS; ++j) {
-              const float s = Pe.x - ys[j];
-              const float t = fmaf(s, s, fmaf(u, beta[j], G + gamma[j]));
-              const bool in = interior || base - (unsigned)(j ^ hs) < (unsigned)(kma - kmi);
-              neg &= in ? __float_as_uint(t) : 0x80000000u;
-            }
-            if (!(neg >> 31)) {  // kk and the exact pre-test are checked in consider
-#pragma unroll
-              for (int j = 0; j < kRS; ++j) {
-                const float s = Pe.x - ys[j];
-                const float t = fmaf(s, s, fmaf(u, beta[j], G + gamma[j]));
-                const bool in = interior || base - (unsigned)(j ^ hs) < (unsigned)(kma - kmi);
-                if (in && !(t < 0.0f)) consider(j, Pe, e);
-              }
-            }
-          }
-          if (improved) atomicMax(best_thr + f, __float_as_uint(bpow));
+      if (__popc(cols) <= __popc(rows)) {
+        do {
+          const int b = __ffs(cols) - 1;
+          cols &= cols - 1;
+          const float2 A = P[s32 + b];
+          if (row) consider(A, swz(s32 + b), Pe, e);
+        } while (cols);
+      } else {
+        do {
+          const int b = __ffs(rows) - 1;
+          rows &= rows - 1;
+          const float2 B = P[e32 + b];
+          if (col) consider(Pi, i, B, swz(e32 + b));
+        } while (rows);
+      }
+      const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(bpow));
+      if (m) {
+        const int k = __reduce_min_sync(0xffffffffu, __float_as_uint(bpow) == m ? bk : INT_MAX);
+        if (lane == 0) {
+          atomicMax(best_thr + f, m);
+          atomicMax(best_key + f, pack_key(__uint_as_float(m), k >> 15, k & 0x7fff));
         }
       }
-      if (s0 >= 0) flush();
     }
   }
   __syncthreads();
@@ -1136,11 +1052,8 @@ int make_plan(uint32_t nb, uint32_t kma, uint32_t nf, uint32_t F_req, Plan *p) {
   uint32_t Tg = (nb + R - 1) / R;
   Tg = (Tg + 31) / 32 * 32;
   if (Tg < 64) Tg = 64;  // at most 8 groups: named barriers 1..8
-  // prefix entries 0 .. nb + kma are written and scan tasks read starts up to nb + kRS - 2;
-  // the prefix array is padded to whole 32-entry chunks, followed by one (max, min) pair
-  // per chunk
-  const uint32_t last = nb + (kma > (uint32_t)kRS ? kma : (uint32_t)kRS);
-  const uint32_t lp = (last + 1 + 31) / 32 * 32;
+  // prefix entries 0 .. nb + kma, padded to whole 32-entry chunks
+  const uint32_t lp = (nb + kma + 1 + 31) / 32 * 32;
   // prefix entries, one float2 (max, min) per chunk, one float (last count) per chunk
   uint32_t region = lp + lp / 32 + (lp / 32 + 1) / 2;
   region = (region + 1) & ~1u;  // 16-byte multiple for the zero fill

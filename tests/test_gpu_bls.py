@@ -154,3 +154,18 @@ def test_concentrated_bins_use_exact_fallback(cuda):
     osr, op1, op2, opmax = oracle.bls(lc, tu, nf, nb, 52, 2, 5, fmin, df)
     _check_spectrum(sr.cpu().numpy(), p1.cpu().numpy(), p2.cpu().numpy(), osr, op1, op2, opmax,
                     lc, tu, dict(nb=nb, fmin=fmin, df=df))
+
+
+@pytest.mark.parametrize("nb,kma,kmi", [(20, 10, 1), (31, 15, 1), (33, 7, 3), (96, 48, 30), (512, 33, 31), (1000, 499, 1),
+                                        (2048, 205, 204), (2048, 64, 1)])
+@pytest.mark.parametrize("n", [1500, 3001])
+def test_scan_chunks_at_their_edges(cuda, n, nb, kma, kmi):
+    """Units of 32 starts by 32 ends: bin counts under, at and off a multiple of 32, windows of one
+    width, of every width and across several chunks, sparse and full bins, a strong transit (few
+    units survive) and none (many do)."""
+    wl = synth.plain_bls(nq=4, n=n, nf=25, nb=nb, seed=nb + n, n_transit=2)
+    lc, tu = torch.from_numpy(wl.lc).to(cuda), torch.from_numpy(wl.tu).to(cuda)
+    sr, p1, p2 = api.geebls_simple(lc, tu, wl.nf, nb, kma, kmi, 1, wl.fmin, wl.df, with_phase=True)
+    osr, op1, op2, opmax = oracle.bls(wl.lc, wl.tu, wl.nf, nb, kma, kmi, 1, wl.fmin, wl.df)
+    _check_spectrum(sr.cpu().numpy(), p1.cpu().numpy(), p2.cpu().numpy(), osr, op1, op2, opmax,
+                    wl.lc, wl.tu, dict(nb=nb, fmin=wl.fmin, df=wl.df))
