@@ -356,10 +356,10 @@ __device__ __forceinline__ unsigned long long pack_key(float pw, int i, int e) {
          (unsigned long long)(0xffffffffu - (((unsigned)i << 15) | (unsigned)e));
 }
 
-// Shared layout of a frequency's histogram / prefix entries (8 bytes each): within every
-// aligned block of 8 entries the slot is XOR-permuted by bits 4..6 of the index, so that a
-// warp whose lanes touch entries 8*lane + r (the prefix pass) spreads over all 16 bank pairs,
-// while 32 consecutive entries still map onto the same aligned 32-entry block.
+// Shared layout of a frequency's prefix entries (8 bytes each; the 64-bit refold's bins too):
+// within every aligned block of 8 entries the slot is XOR-permuted by bits 4..6 of the index, so
+// that a warp whose lanes write entries 8*lane + r (the prefix pass) spreads over all 16 bank
+// pairs, while 32 consecutive entries still map onto the same aligned 32-entry block.
 __device__ __forceinline__ int swz(int e) { return e ^ ((e >> 4) & 7); }
 
 // int64 -> float off the FP64 pipe (the 64-bit conversion issues there, and that pipe is
@@ -407,19 +407,23 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
   const int tid = threadIdx.x;
   const int nb = (int)a.nb;
 
-  // zero the histograms
-  {
-    ulonglong2 *z = reinterpret_cast<ulonglong2 *>(sm);
-    const uint32_t nz = (a.F * a.region) / 2;
-    for (uint32_t k = tid; k < nz; k += kThreads) z[k] = make_ulonglong2(0ull, 0ull);
-    if (tid < 64) drop_cnt[tid] = 0u;
+  // zero the histograms: nbp words S and nbp words C a frequency
+  const uint32_t nbp = ((uint32_t)nb + 15u) & ~15u;
+  for (uint32_t f = 0; f < nfrem; ++f) {
+    ulonglong2 *z = reinterpret_cast<ulonglong2 *>(sm + (size_t)f * a.region);
+    for (uint32_t k = tid; k < nbp / 2; k += kThreads) z[k] = make_ulonglong2(0ull, 0ull);
   }
+  if (tid < 64) drop_cnt[tid] = 0u;
   __syncthreads();
 
   // ---- fold.  Fast format: two 32-bit words per bin, S += xq >> 10 and
   // C += ((xq & 1023) << 12) | 1, exact while every bin holds at most kFastMaxCount
   // samples (|xq| < 2^30).  The scan verifies that and re-folds a frequency in the 64-bit
-  // format ((xq << CB) | 1, one 64-bit atomic) when it does not hold.
+  // format ((xq << CB) | 1, one 64-bit atomic) when it does not hold.  The words S of all bins lie
+  // first, then the words C, both in bin order: an update needs no index arithmetic beyond its
+  // bin, and a warp's 32 samples, evenly spaced in phase, meet in a bank least often (model of
+  // 29.4-min and 2-min cadences: 2.37 and 2.00 conflict wavefronts an atomic; words of a bin side
+  // by side, eight-bin blocks permuted for the prefix pass's reads: 2.91 and 2.29).
   const int32_t *Xq = tj.X;
   const int CB = tj.CB;
   unsigned *h32 = reinterpret_cast<unsigned *>(sm);
@@ -460,13 +464,10 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
           const unsigned wS = (unsigned)(xq[u] >> 10);
           const unsigned wC = ((unsigned)(xq[u] & 1023) << 12) | 1u;
           unsigned long long ph = ab[u].x + (unsigned long long)j0 * ab[u].y;
-          // S in the low word for bins with bit 4 clear, in the high word otherwise, so that
-          // the S (and the C) updates of a warp reach all 32 banks
           auto add = [&](unsigned *h) {
             const uint32_t bin = MODE == 0 ? (uint32_t)(ph >> shift) : (uint32_t)__umul64hi(ph, (unsigned long long)nb);
-            const uint32_t w = 2u * (uint32_t)swz((int)bin) + ((bin >> 4) & 1u);
-            atomicAdd(h + w, wS);
-            atomicAdd(h + (w ^ 1u), wC);
+            atomicAdd(h + bin, wS);
+            atomicAdd(h + nbp + bin, wC);
             ph += ab[u].y;
           };
           if constexpr (NF > 0) {
@@ -500,9 +501,8 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
       for (uint32_t f = 0; f < nfrem; ++f) {
         const uint32_t bin = ref_bin(t, f);
         if (bin < (uint32_t)nb) {
-          const uint32_t w = 2u * (uint32_t)swz((int)bin) + ((bin >> 4) & 1u);
-          atomicAdd(h + w, wS);
-          atomicAdd(h + (w ^ 1u), wC);
+          atomicAdd(h + bin, wS);
+          atomicAdd(h + nbp + bin, wC);
         } else {
           atomicAdd(drop_cnt + f, 1u);
         }
@@ -559,13 +559,24 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
     int scv = 0, ec = 0, tc = 0;
     for (int pass = 0; pass < 2; ++pass) {
       const bool fast = pass == 0;
-      unsigned long long hv[R];
+      uint32_t hs[R], hc[R];   // this thread's bins: words S and C, or low and high words
+      if (fast) {
+        const uint4 *S4 = reinterpret_cast<const uint4 *>(H), *C4 = reinterpret_cast<const uint4 *>(h32 + 2 * (size_t)f * a.region + nbp);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int b = i0 + r;
-        unsigned long long v = b < nb ? H[swz(b)] : 0ull;
-        if (fast && ((b >> 4) & 1)) v = (v << 32) | (v >> 32);  // S back in the low word
-        hv[r] = v;
+        for (int r = 0; r < R; r += 4) {  // bins past nb are zero up to nbp
+          const bool in = i0 + r < (int)nbp;
+          const uint4 u = in ? S4[(i0 + r) >> 2] : make_uint4(0u, 0u, 0u, 0u);
+          const uint4 v = in ? C4[(i0 + r) >> 2] : make_uint4(0u, 0u, 0u, 0u);
+          hs[r] = u.x; hs[r + 1] = u.y; hs[r + 2] = u.z; hs[r + 3] = u.w;
+          hc[r] = v.x; hc[r + 1] = v.y; hc[r + 2] = v.z; hc[r + 3] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const unsigned long long v = i0 + r < nb ? H[swz(i0 + r)] : 0ull;
+          hs[r] = (uint32_t)v;
+          hc[r] = (uint32_t)(v >> 32);
+        }
       }
       group_bar(1 + g, Tg);
       sxv = 0;
@@ -576,11 +587,12 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
         long long xs;
         int c;
         if (fast) {
-          xs = (long long)(int)(unsigned)(hv[r] & 0xffffffffull) * 1024 + (long long)(hv[r] >> 44);
-          c = (int)((hv[r] >> 32) & 0xfffull);
+          xs = (long long)(int)hs[r] * 1024 + (long long)(hc[r] >> 12);
+          c = (int)(hc[r] & 0xfffu);
         } else {
-          xs = (long long)hv[r] >> CB;
-          c = (int)(hv[r] & cmask);
+          const unsigned long long v = ((unsigned long long)hc[r] << 32) | hs[r];
+          xs = (long long)v >> CB;
+          c = (int)(v & cmask);
         }
         sxv += xs;
         scv += c;
@@ -620,7 +632,7 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
       group_bar(1 + g, Tg);  // every thread has read scan_* and H before they are rewritten
       {
         ulonglong2 *z = reinterpret_cast<ulonglong2 *>(H);
-        for (uint32_t k = gtid; k < a.region / 2; k += Tg) z[k] = make_ulonglong2(0ull, 0ull);
+        for (uint32_t k = gtid; k < nbp / 2; k += Tg) z[k] = make_ulonglong2(0ull, 0ull);
       }
       group_bar(1 + g, Tg);
       refold64(f, gtid, Tg);
