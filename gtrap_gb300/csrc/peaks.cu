@@ -277,6 +277,429 @@ __global__ void __launch_bounds__(kPkThreads) peakstat_kernel(
   if (tid == 0) out[q] = r;
 }
 
+// ---- series that fit in shared memory
+
+constexpr int kStThreads = 1024;
+constexpr int kStBins = 2048;   // digits of 11 + 11 + 10 bits
+
+struct StScratch {
+  float part[3][kStThreads / 32];
+  float m0;
+  unsigned wsum[kStThreads / 32];
+  unsigned wkey[2][kStThreads / 32], widx[2][kStThreads / 32];
+  unsigned digit, below, count, vmin;
+};
+
+// A sum of floats as three floats (error-free transformations; about 70 bits).  The FP64 pipe of
+// this part takes a warp's 32 additions in 16 cycles or more, so the long sums run on FP32 and only
+// their totals are joined in FP64.
+struct Sum3 {
+  float a = 0.0f, b = 0.0f, c = 0.0f;
+  static __device__ __forceinline__ float two_sum(float x, float y, float &e) {
+    const float s = __fadd_rn(x, y), t = __fsub_rn(s, x);
+    e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, t)), __fsub_rn(y, t));
+    return s;
+  }
+  __device__ __forceinline__ void add(float v) {
+    float e1, e2;
+    a = two_sum(a, v, e1);
+    b = two_sum(b, e1, e2);
+    c = __fadd_rn(c, e2);
+  }
+  __device__ __forceinline__ void add(const Sum3 &o) { add(o.a); add(o.b); add(o.c); }
+  __device__ __forceinline__ void add_product(float x, float y) {   // x y exactly
+    const float p = __fmul_rn(x, y);
+    add(p);
+    add(__fmaf_rn(x, y, -p));
+  }
+  __device__ __forceinline__ void over_warp() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      Sum3 u;
+      u.a = __shfl_xor_sync(0xffffffffu, a, o);
+      u.b = __shfl_xor_sync(0xffffffffu, b, o);
+      u.c = __shfl_xor_sync(0xffffffffu, c, o);
+      // the same order on both sides of an exchange: every lane gets the same total
+      Sum3 lo = threadIdx.x & o ? u : *this;
+      lo.add(threadIdx.x & o ? *this : u);
+      *this = lo;
+    }
+  }
+};
+
+// the block's total, on warp 0 (all its lanes)
+__device__ __forceinline__ Sum3 st_total(Sum3 v, StScratch &sc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v.over_warp();
+  __syncthreads();
+  if (lane == 0) { sc.part[0][warp] = v.a; sc.part[1][warp] = v.b; sc.part[2][warp] = v.c; }
+  __syncthreads();
+  Sum3 w;
+  if (warp == 0) {
+    w.a = sc.part[0][lane]; w.b = sc.part[1][lane]; w.c = sc.part[2][lane];
+    w.over_warp();
+  }
+  return w;
+}
+
+// Population standard deviation of the val(e), e < n, with use(e) (count of them, at least one),
+// from the deviations about the mean's float; on thread 0.
+template <typename Val, typename Use>
+__device__ __forceinline__ double st_std(Val val, Use use, unsigned n, unsigned count, StScratch &sc) {
+  const int tid = threadIdx.x;
+  // a power of two out of the squares' way: the largest magnitude times 2^-ex is below 4
+  __syncthreads();
+  if (tid == 0) sc.vmin = 0u;
+  __syncthreads();
+  unsigned big = 0u;
+  for (unsigned e = tid; e < n; e += kStThreads)
+    if (use(e)) big = max(big, __float_as_uint(fabsf(val(e))));
+  big = __reduce_max_sync(0xffffffffu, big);
+  if ((tid & 31) == 0) atomicMax(&sc.vmin, big);
+  __syncthreads();
+  const float vbig = __uint_as_float(sc.vmin);
+  const int ex = isfinite(vbig) && vbig > 0.0f ? min(max(ilogbf(vbig), -126), 126) : 0;
+  const float down = ldexpf(1.0f, -ex);
+  Sum3 s;
+  for (unsigned e = tid; e < n; e += kStThreads)
+    if (use(e)) s.add(__fmul_rn(val(e), down));
+  const Sum3 all = st_total(s, sc);
+  double total = 0.0;
+  if (tid == 0) {   // (FP64 on one warp only: a division takes a warp hundreds of cycles here)
+    total = (double)all.a + ((double)all.b + (double)all.c);
+    sc.m0 = (float)(total / (double)count);
+  }
+  __syncthreads();
+  const float m0 = sc.m0;
+  Sum3 ss;
+  for (unsigned e = tid; e < n; e += kStThreads) {
+    if (!use(e)) continue;
+    float lo;
+    const float d = Sum3::two_sum(__fmul_rn(val(e), down), -m0, lo);   // value - m0 = d + lo exactly
+    ss.add_product(d, d);
+    ss.add_product(d, __fadd_rn(lo, lo));
+    ss.add(__fmul_rn(lo, lo));
+  }
+  const Sum3 sq = st_total(ss, sc);
+  double std = 0.0;
+  if (tid == 0) {
+    const double dev = total - (double)count * (double)m0;   // sum of the deviations from m0
+    const double var = ((double)sq.a + ((double)sq.b + (double)sq.c) - dev * dev / (double)count) / (double)count;
+    std = ldexp(sqrt(var <= 0.0 ? 0.0 : var), ex);
+  }
+  return std;
+}
+
+// exclusive prefix over the block's threads; the total in sc.count
+__device__ __forceinline__ unsigned st_scan(unsigned c, StScratch &sc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  __syncthreads();
+  if (lane == 31) sc.wsum[warp] = incl;
+  __syncthreads();
+  const unsigned w = sc.wsum[lane];
+  const unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
+  const unsigned all = __reduce_add_sync(0xffffffffu, w);
+  if (threadIdx.x == 0) sc.count = all;
+  return before + incl - c;
+}
+
+// the k-th and (k + step)-th smallest (0-based, step 0 or 1) of val(0 .. n): radix selection over
+// three digits of the order-preserving keys; the next larger value by one more pass if it is not
+// the same one
+template <typename Val>
+__device__ __forceinline__ void st_select(Val val, unsigned n, unsigned k, unsigned step, unsigned *hist,
+                                          StScratch &sc, float &a, float &b) {
+  const int tid = threadIdx.x;
+  auto key_of = [](float v) { return isnan(v) ? 0u : okey(v); };   // NaN ranks lowest
+  unsigned prefix = 0, mask = 0, left = k, same = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int shift = d == 0 ? 21 : d == 1 ? 10 : 0;
+    const unsigned bins = d == 2 ? 1024u : 2048u;
+    __syncthreads();
+    hist[tid] = 0;
+    hist[tid + kStThreads] = 0;
+    __syncthreads();
+    for (unsigned e = tid; e < n; e += kStThreads) {
+      const unsigned u = key_of(val(e));
+      if ((u & mask) == prefix) atomicAdd(hist + ((u >> shift) & (bins - 1)), 1u);
+    }
+    __syncthreads();
+    const unsigned c0 = hist[2 * tid], c1 = hist[2 * tid + 1];
+    const unsigned before = st_scan(c0 + c1, sc);
+    if (left >= before && left < before + c0) { sc.digit = 2 * tid; sc.below = before; sc.vmin = c0; }
+    if (left >= before + c0 && left < before + c0 + c1) { sc.digit = 2 * tid + 1; sc.below = before + c0; sc.vmin = c1; }
+    __syncthreads();
+    prefix |= sc.digit << shift;
+    mask |= (bins - 1) << shift;
+    left -= sc.below;
+    same = sc.vmin;
+  }
+  a = okey_inv(prefix);
+  b = a;
+  if (left + step >= same) {   // the next value is a larger one (uniform)
+    __syncthreads();
+    if (tid == 0) sc.vmin = 0xffffffffu;
+    __syncthreads();
+    unsigned m = 0xffffffffu;
+    for (unsigned e = tid; e < n; e += kStThreads) {
+      const unsigned u = key_of(val(e));
+      if (u > prefix) m = min(m, u);
+    }
+    m = __reduce_min_sync(0xffffffffu, m);
+    if ((tid & 31) == 0) atomicMin(&sc.vmin, m);
+    __syncthreads();
+    b = okey_inv(sc.vmin);
+  }
+}
+
+// peakstat_kernel for series that fit (staged_max(): about 35,000 samples): the series is copied
+// to shared memory once (a column of an [n, nq] image touches a sector a sample, so each of the
+// passes below cost 32 bytes a sample out of L2 before), candidates become a list in index order
+// and the suppression, the highest peaks and the statistics of the rest run over lists.  Latency
+// bound (block-wide steps over a few samples a thread): 96 series of 18,000 samples 815 -> 81 us,
+// of which the copy takes 10, the suppression's 8 rounds 10 and the two deviations 20.
+__global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
+    const float *__restrict__ x, const unsigned long long *__restrict__ off,
+    const uint32_t *__restrict__ len, size_t stride, uint32_t max_n, uint32_t mpd, uint32_t ntop, uint32_t k,
+    gtrap_peak_stats *out, uint32_t *peak_idx, float *peak_val) {
+  extern __shared__ __align__(16) float sv[];     // [max_n] the series
+  // candidates' states as bits (a word and a zero word on either side), their positions, and the
+  // kept peaks' positions (while the suppression runs: the masks of higher candidates)
+  const unsigned words = max_n / 64 + 3;
+  volatile unsigned *und = reinterpret_cast<unsigned *>(sv + max_n) + 1;
+  volatile unsigned *kep = und + words;
+  unsigned short *list = reinterpret_cast<unsigned short *>(sv + max_n) + 4 * words;   // [max_n / 2 + 1]
+  unsigned short *kept = list + max_n / 2 + 1;                                          // [max_n / 2 + 1]
+  __shared__ unsigned hist[kStBins];
+  __shared__ StScratch sc;
+  const int q = blockIdx.x, tid = threadIdx.x;
+  const int n = (int)len[q];
+  {
+    const float *src = x + off[q];
+    for (int e = tid; e < n; e += kStThreads) {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(sv + e);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src + (size_t)e * stride) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncthreads();
+  gtrap_peak_stats r;
+  r.argmax = 0; r.lent = 0; r.npeaks = 0;
+  r.maxsn = 0.0f; r.median = 0.0; r.std = 0.0; r.far = 0.0; r.pssn = INFINITY; r.diff = 0.0;
+  r.medc = 0.0; r.stdc = 0.0;
+
+  // ---- max / argmax (NaN wins, as np.max propagates it; then the larger value, then the lower
+  // index), positive count and sum; candidates, counted and then listed in index order: a thread
+  // takes a run of samples (an odd number: no bank conflicts)
+  const int run = ((n + kStThreads - 1) / kStThreads) | 1;
+  const int e0 = min(n, tid * run), e1 = min(n, e0 + run);
+  auto candidate = [&](int e) {
+    if (e < 1 || e + 1 >= n) return false;
+    const float a = sv[e - 1], v = sv[e], c = sv[e + 1];
+    return !isnan(a) && !isnan(v) && !isnan(c) && v > a && !(c > v);
+  };
+  // the highest key, then the lowest index (largest complement) of it, over the block; buffer `w`
+  auto block_best = [&](unsigned key, unsigned idx, int w) -> uint2 {
+    const unsigned m = __reduce_max_sync(0xffffffffu, key);
+    const unsigned i = __reduce_max_sync(0xffffffffu, key == m ? idx : 0u);
+    if ((tid & 31) == 0) { sc.wkey[w][tid >> 5] = m; sc.widx[w][tid >> 5] = i; }
+    __syncthreads();
+    const unsigned km = sc.wkey[w][tid & 31], ki = sc.widx[w][tid & 31];
+    const unsigned bm = __reduce_max_sync(0xffffffffu, km);
+    return make_uint2(bm, __reduce_max_sync(0xffffffffu, km == bm ? ki : 0u));
+  };
+  unsigned pcnt = 0, ncand = 0;
+  uint2 top;
+  {
+    float vmax = -INFINITY;
+    int imax = INT_MAX;
+    for (int e = e0; e < e1; ++e) {
+      const float v = sv[e];
+      if (v > vmax || (v == vmax && e < imax) || (isnan(v) && !isnan(vmax))) { vmax = v; imax = e; }
+      pcnt += v > 0.0f ? 1u : 0u;
+      ncand += candidate(e) ? 1u : 0u;
+    }
+    const bool any = imax != INT_MAX;
+    top = block_best(!any ? 0u : isnan(vmax) ? 0xffffffffu : okey(vmax), any ? 0xffffffffu - (unsigned)imax : 0u, 0);
+  }
+  unsigned at = st_scan(ncand, sc);
+  for (int e = e0; e < e1; ++e)
+    if (candidate(e)) list[at++] = (unsigned short)e;
+  __syncthreads();
+  const int M = (int)sc.count;
+  if (top.y) {
+    r.argmax = 0xffffffffu - top.y;
+    r.maxsn = sv[r.argmax];
+  }
+  __syncthreads();
+  st_scan(pcnt, sc);
+  __syncthreads();
+  r.lent = sc.count;
+  r.std = NAN;
+  // population std of the positive values, median of all; r's FP64 members are thread 0's alone
+  if (r.lent > 0)
+    r.std = st_std([&](unsigned e) { return sv[e]; }, [&](unsigned e) { return sv[e] > 0.0f; }, (unsigned)n, r.lent, sc);
+  if (n > 0) {
+    float m1, m2;
+    st_select([&](unsigned e) { return sv[e]; }, (unsigned)n, (unsigned)(n - 1) / 2, n % 2 ? 0u : 1u, hist, sc, m1, m2);
+    if (tid == 0) r.median = 0.5 * ((double)m1 + (double)m2);
+  }
+  if (tid == 0) r.far = ((double)r.maxsn - r.median) / r.std;
+
+  // ---- greedy suppression within +-mpd, in rounds over the list, a warp taking 32 candidates, one
+  // word of each state, at a time.  Only a candidate of higher priority can delete or hold up
+  // another, and candidates are never adjacent: for windows of up to 16 samples the higher ones among
+  // the eight entries on either side are found once, as a mask, and a round compares it with the
+  // states' bits there; wider windows look at their entries one by one
+  const int w = (int)mpd, lane = tid & 31;
+  const int nword = (M + 31) >> 5;
+  const bool masks = w > 0 && w <= 16;
+  unsigned short *higher = kept;   // bit j: entry c - 8 + j (j < 8) or c - 7 + j
+  if (tid < 2) { const int i = tid ? nword : -1; und[i] = 0u; kep[i] = 0u; }
+  for (int i = tid >> 5; i < nword; i += kStThreads / 32) {
+    const int c = 32 * i + lane;
+    unsigned m = w > 0 ? 1u : 0u;
+    if (masks && c < M) {
+      const int e = list[c];
+      const float v = sv[e];
+      m = 0u;
+      for (int d = 1; d <= w / 2; ++d) {   // the d-th entry on either side is 2d samples away at least
+        const int p = c >= d ? (int)list[c - d] : -70000, s2 = c + d < M ? (int)list[c + d] : 200000;
+        if (e - p <= w && prio_gt(sv[p], p, v, e)) m |= 1u << (8 - d);
+        if (s2 - e <= w && prio_gt(sv[s2], s2, v, e)) m |= 1u << (7 + d);
+      }
+      higher[c] = (unsigned short)m;
+    }
+    const unsigned u = __ballot_sync(0xffffffffu, c < M && m), k0 = __ballot_sync(0xffffffffu, c < M && !m);
+    if (lane == 0) { und[i] = u; kep[i] = k0; }
+  }
+  __syncthreads();
+  if (w > 0) {
+    for (int round = 0; round <= M; ++round) {
+      int busy = 0;
+      for (int i = tid >> 5; i < nword; i += kStThreads / 32) {
+        const unsigned U = und[i];
+        if (!U) continue;
+        const bool mine = (U >> lane) & 1u;
+        bool del = false, blocked = false;
+        const int c = 32 * i + lane;
+        if (masks) {
+          const unsigned m = mine ? higher[c] : 0u;
+          auto around = [&](volatile unsigned *b, unsigned mid) {   // bits of the entries either side
+            const unsigned long long lo = ((unsigned long long)mid << 32) | b[i - 1];
+            const unsigned long long hi = ((unsigned long long)b[i + 1] << 32) | mid;
+            return ((unsigned)(lo >> (24 + lane)) & 0xffu) | (((unsigned)(hi >> (lane + 1)) & 0xffu) << 8);
+          };
+          blocked = m & around(und, U);
+          del = m & around(kep, kep[i]);
+        } else if (mine) {
+          const int e = list[c];
+          const float v = sv[e];
+          auto look = [&](int j) {   // false: past the window
+            const int p = list[j];
+            if (abs(p - e) > w) return false;
+            const unsigned bit = 1u << (j & 31);
+            if (und[j >> 5] & bit) blocked |= prio_gt(sv[p], p, v, e);
+            else if (kep[j >> 5] & bit) del = true;
+            return true;
+          };
+          for (int j = c - 1; j >= 0 && !del && look(j); --j) {}
+          for (int j = c + 1; j < M && !del && look(j); ++j) {}
+        }
+        const unsigned kb = __ballot_sync(0xffffffffu, mine && !del && !blocked);
+        const unsigned db = __ballot_sync(0xffffffffu, mine && del);
+        if (lane == 0) {   // kept before no longer undecided: nobody sees it as deleted in between
+          kep[i] = kep[i] | kb;
+          __threadfence_block();
+          und[i] = U & ~(kb | db);
+        }
+        busy |= (U & ~(kb | db)) != 0u;
+      }
+      if (!__syncthreads_or(busy)) break;
+    }
+  }
+  __syncthreads();
+  // the kept peaks as a list of their own, in index order
+  {
+    unsigned cnt = 0;
+    for (int i = tid; i < nword; i += kStThreads) cnt += __popc(kep[i]);   // (nword <= threads)
+    unsigned to = st_scan(cnt, sc);
+    for (int i = tid; i < nword; i += kStThreads)
+      for (unsigned m = kep[i]; m; m &= m - 1) kept[to++] = list[32 * i + __ffs(m) - 1];
+  }
+  __syncthreads();
+  const unsigned K = sc.count;
+  r.npeaks = K;
+  __syncthreads();
+
+  // ---- the highest peaks in priority order
+  const uint32_t kk = max(k, ntop);
+  float lv = INFINITY;  // last selected peak (value, index): the next one ranks below it
+  int li = -1;
+  float top0 = 0.0f, topn = 0.0f;
+  int topn_i = -1;
+  for (uint32_t t = 0; t < kk && t < K; ++t) {
+    unsigned key = 0u, idx = 0u;
+    for (unsigned c = tid; c < K; c += kStThreads) {
+      const int e = kept[c];
+      const float v = sv[e];
+      if (!prio_gt(lv, li, v, e)) continue;  // already selected
+      const unsigned kv = okey(v), ki = 0xffffffffu - (unsigned)e;
+      if (kv > key || (kv == key && ki > idx)) { key = kv; idx = ki; }
+    }
+    const uint2 b = block_best(key, idx, t & 1);   // (the other buffer's reads ended a barrier ago)
+    li = (int)(0xffffffffu - b.y);
+    lv = okey_inv(b.x);
+    if (t == 0) top0 = lv;
+    if (t + 1 == ntop) { topn = lv; topn_i = li; }
+    if (tid == 0 && t < k) {
+      peak_idx[(size_t)q * k + t] = (uint32_t)li;
+      peak_val[(size_t)q * k + t] = lv;
+    }
+  }
+  if (tid == 0)
+    for (uint32_t t = min(K, k); t < k; ++t) {
+      peak_idx[(size_t)q * k + t] = 0xffffffffu;
+      peak_val[(size_t)q * k + t] = 0.0f;
+    }
+
+  // ---- statistics of the peaks after the ntop highest
+  if (ntop > 0 && K > ntop) {
+    const uint32_t m = K - ntop;
+    auto rest = [&](int e) { return prio_gt(topn, topn_i, sv[e], e); };
+    r.stdc = st_std([&](unsigned c) { return sv[kept[c]]; }, [&](unsigned c) { return rest(kept[c]); }, K, m, sc);
+    // the rest are the K - ntop lowest of the kept: ranks of the rest are ranks of them all
+    float c1, c2;
+    st_select([&](unsigned c) { return sv[kept[c]]; }, K, (m - 1) / 2, m % 2 ? 0u : 1u, hist, sc, c1, c2);
+    if (tid == 0) {
+      r.medc = 0.5 * ((double)c1 + (double)c2);
+      r.pssn = ((double)top0 - r.medc) / r.stdc;
+      r.diff = ((double)topn - r.median) / r.std;
+    }
+  }
+  if (tid == 0) out[q] = r;
+}
+
+// Shared memory of a staged series: values, states and two lists of positions (candidates are
+// never adjacent, so at most half as many as samples).
+size_t staged_bytes(size_t max_n) { return 4 * max_n + 8 * (max_n / 64 + 3) + 4 * (max_n / 2 + 1); }
+
+size_t staged_max() {
+  const size_t room = (size_t)gtrap::max_smem_optin() - sizeof(StScratch) - kStBins * sizeof(unsigned) - 256;
+  size_t n = room / 6;
+  // positions are 16-bit, and a thread lists the kept of one word of states
+  if (n > 64 * kStThreads - 64) n = 64 * kStThreads - 64;
+  while (n && staged_bytes(n) > room) --n;
+  return n;
+}
+
 }  // namespace
 
 extern "C" {
@@ -299,6 +722,13 @@ int gtrap_peakstat(const float *sn, const uint64_t *off, const uint32_t *n, uint
   if (smem > gtrap_peakstat_max_samples())
     return fail(GTRAP_ERR_UNSUPPORTED, "peakstat: series of %u samples exceed the %zu that fit in shared memory",
                 max_n, gtrap_peakstat_max_samples());
+  if (smem <= staged_max()) {
+    const size_t bytes = staged_bytes(smem);
+    GTRAP_TRY(ensure_smem((const void *)peakstat_staged_kernel, bytes, "peakstat"));
+    peakstat_staged_kernel<<<ncurves, kStThreads, bytes, stream>>>(sn, (const unsigned long long *)off, n, (size_t)stride,
+                                                                  (uint32_t)smem, mpd, ntop, k, stats, peak_idx, peak_val);
+    return check_launch("peakstat_staged_kernel");
+  }
   GTRAP_TRY(ensure_smem((const void *)peakstat_kernel, smem, "peakstat"));
   peakstat_kernel<<<ncurves, kPkThreads, smem, stream>>>(sn, (const unsigned long long *)off, n,
                                                          (size_t)stride, mpd, ntop, k, stats,

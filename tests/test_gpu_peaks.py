@@ -83,3 +83,37 @@ def test_peakstat_of_packed_batch(cuda):
     st = api.stats_to_numpy(st)
     for q in range(bat.n_tls):
         _check(st[q], idx.cpu().numpy()[q], val.cpu().numpy()[q], bat.tls_result(q)[0], 10, 4, 6)
+
+
+@pytest.mark.parametrize("mpd,ntop,k", [(10, 4, 8), (0, 2, 5), (1, 3, 4), (1000, 1, 2)])
+def test_staged_and_long_series_agree(cuda, mpd, ntop, k):
+    """Series that fit in shared memory run on one kernel, a launch with a longer one on another:
+    the same series through both, with NaN, infinities, constants, ramps, every sample a peak and
+    the shortest lengths.  Counts, indices, heights and order statistics equal; the FP64 sums
+    differ by their order only."""
+    rng = np.random.default_rng(11)
+    xs = [_series(j) for j in range(3)]
+    y = rng.normal(size=4097).astype(np.float32)
+    y[[5, 100, 4096]] = np.nan
+    y[200:203] = np.inf
+    y[300] = -np.inf
+    xs += [y, np.zeros(50, np.float32), np.arange(3000, dtype=np.float32), np.arange(3000, 0, -1).astype(np.float32),
+           np.tile([0, 1], 1500).astype(np.float32), np.ones(1, np.float32), np.ones(2, np.float32),
+           np.array([0, 2, 1], np.float32), rng.normal(size=30000).astype(np.float32), -np.ones(9, np.float32)]
+
+    def run(series):
+        lens = np.array([x.size for x in series])
+        offs = np.concatenate([[0], np.cumsum(lens)[:-1]])
+        st, idx, val = api.peakstat(torch.from_numpy(np.concatenate(series)).to(cuda),
+                                    torch.from_numpy(offs.astype(np.int64)).to(cuda),
+                                    torch.from_numpy(lens.astype(np.int32)).to(cuda), 1, int(lens.max()), mpd, ntop, k)
+        return api.stats_to_numpy(st), idx.cpu().numpy(), val.cpu().numpy()
+
+    a, ai, av = run(xs)
+    b, bi, bv = run(xs + [np.zeros(60000, np.float32)])
+    np.testing.assert_array_equal(ai, bi[:-1])
+    np.testing.assert_array_equal(av, bv[:-1])
+    for key in STAT_KEYS + ("medc",):
+        np.testing.assert_array_equal(a[key], b[key][:-1], err_msg=key)
+    for key in ("std", "far", "pssn", "diff", "stdc"):
+        np.testing.assert_allclose(a[key], b[key][:-1], rtol=1e-11, atol=1e-13, err_msg=key)
