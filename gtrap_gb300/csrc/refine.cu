@@ -32,7 +32,8 @@ using gtrap::frac64;
 constexpr int kThreads = 256;
 constexpr int kMaxFine = 4096;        // fine bins of one neighbourhood, (p2 - p1 + 1 + 2M) * S
 constexpr double kXqMax = 1099511627776.0;  // |quantised flux| < 2^40
-constexpr int kMaxGroup = 16;               // trials per block at most
+constexpr int kMaxGroup = 33;               // trials per block at most
+constexpr int kFineMax = 2047;              // samples a fine bin's 32-bit words hold
 constexpr size_t kSmemBudget = 96 * 1024;   // fine histograms of one block (two blocks per SM)
 
 // One trial frequency's best window (and the curve's constants every block recomputes).
@@ -45,6 +46,17 @@ struct Part {
   uint32_t j, p1;       // grid peak and its start bin
   int32_t sx;           // flux scale exponent
   float tref;           // middle of the valid time span (float32)
+};
+
+// What every trial of a curve shares, from one block a curve: the grid peak, its neighbourhood, the
+// flux scale and the reference time.  (Every block of trials found them again before, from the whole
+// spectrum and the whole curve.)
+struct Head {
+  uint32_t j, p1, L, M;   // grid peak, its start bin, coarse bins and margin of the neighbourhood
+  uint32_t nv;            // valid samples
+  int32_t sx;             // flux scale exponent
+  float tref;             // middle of the valid time span (float32)
+  int32_t ok;             // 0: no refinement
 };
 
 struct RefCurve {
@@ -64,9 +76,10 @@ struct RefArgs {
   uint32_t n, nq, nf, kkmi;
   float fmin, df;
   uint32_t nb, kma, kmi, K, S, M;
-  uint32_t G;                     // trials per block
+  uint32_t smem, min_groups;      // a block's dynamic shared memory, groups of trials a curve at least
   int lognb, logK;
   Part *part;                     // [count, 2K + 1]
+  Head *head;                     // [count]
   gtrap_bls_refined *out;
 };
 
@@ -93,28 +106,24 @@ __device__ __forceinline__ bool valid(float t, float x) {
 
 // rint((x - off) * 2^sx) for finite floats with |x - off| * 2^sx < 2^40 (at most one unit off
 // the exact rounding), in FP32 and integer instructions: x - off = s + e exactly (TwoSum),
-// s * 2^sx split into 20-bit halves.
-__device__ __forceinline__ long long quantise(float x, float off, int sx) {
+// s * 2^sx split into 20-bit halves.  2^sx comes as two factors (either may be out of the float
+// range as one); scaling up is exact, and what scaling down rounds is below one unit.
+struct Scale {
+  float a, b;
+  __device__ explicit Scale(int sx) : a(ldexpf(1.0f, sx / 2)), b(ldexpf(1.0f, sx - sx / 2)) {}
+};
+
+__device__ __forceinline__ long long quantise(float x, float off, const Scale &sc) {
   const float s = __fsub_rn(x, off);
   const float bv = __fsub_rn(s, x);
   const float e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, bv)), __fsub_rn(-off, bv));
-  const float S = ldexpf(s, sx), Es = ldexpf(e, sx);
-  const float hi = truncf(ldexpf(S, -20));
-  const float lo = __fsub_rn(S, ldexpf(hi, 20));  // exact: S with its top bits removed
+  const float S = __fmul_rn(__fmul_rn(s, sc.a), sc.b), Es = __fmul_rn(__fmul_rn(e, sc.a), sc.b);
+  const float hi = truncf(__fmul_rn(S, 0x1p-20f));
+  const float lo = __fsub_rn(S, __fmul_rn(hi, 0x1p20f));  // exact: S with its top bits removed
   return ((long long)__float2int_rz(hi) << 20) + (long long)__float2int_rn(lo) + (long long)__float2int_rn(Es);
 }
 
-// Block reductions (kThreads threads); every thread gets the result.
-__device__ float block_max(float v, float *sh) {
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  v = sh[0];
-  for (int w = 1; w < kThreads / 32; ++w) v = fmaxf(v, sh[w]);
-  return v;
-}
-
+// Block reduction (kThreads threads); every thread gets the result.
 template <typename T>
 __device__ T block_sum(T v, T *sh) {  // fixed order: lanes by shuffle tree, warps in order
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -131,237 +140,371 @@ __device__ __forceinline__ bool better(double p, uint32_t a, uint32_t b, double 
   return p > bp || (p == bp && (a < ba || (a == ba && b < bb)));
 }
 
-// One block per (curve, group of G consecutive trials): the samples are read and their exact
-// phase pairs formed once for the group, and each trial gets its own fine histogram.
-__global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a) {
-  extern __shared__ __align__(16) unsigned char dyn[];
-  __shared__ float shf[kThreads / 32];
-  __shared__ long long shl[kThreads / 32];
-  __shared__ unsigned shu[kThreads / 32];
-  __shared__ uint32_t sj;
-  __shared__ float pmax_s[kMaxGroup];
+constexpr int kHeadThreads = 512;
+
+__global__ void __launch_bounds__(kHeadThreads) refine_head_kernel(const RefArgs a) {
+  constexpr int kW = kHeadThreads / 32, kU = 8;
+  __shared__ float shf[4][kW];
+  __shared__ uint32_t shn[kW], sj;
   const uint32_t c = blockIdx.x;
-  const uint32_t nk_all = 2 * a.K + 1;
-  const uint32_t k0 = blockIdx.y * a.G;
-  const uint32_t nk = min(a.G, nk_all - k0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const RefCurve cv = curve_of(a, c);
-  Part *pt = a.part + (size_t)c * nk_all + k0;
-
-  // ---- grid peak: first maximum of the spectrum
+  // grid peak: first maximum of the spectrum
   float best = -INFINITY;
   uint32_t bj = UINT_MAX;
-  for (uint32_t j = tid; j < cv.nf; j += kThreads) {
-    const float v = a.blsp[cv.out + j];
-    if (v > best) { best = v; bj = j; }  // strided ascending j: the first maximum of this thread
+  for (uint32_t j0 = 0; j0 < cv.nf; j0 += kHeadThreads * kU) {   // kU loads ahead of their uses
+    float v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t j = j0 + u * kHeadThreads + tid;
+      v[u] = j < cv.nf ? __ldg(a.blsp + cv.out + j) : -INFINITY;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (v[u] > best) { best = v[u]; bj = j0 + u * kHeadThreads + tid; }  // ascending: this thread's first maximum
   }
-  const float gmax = block_max(best, shf);
-  if (tid == 0) sj = UINT_MAX;
-  __syncthreads();
-  if (best == gmax && bj != UINT_MAX) atomicMin(&sj, bj);
-  __syncthreads();
-  const uint32_t j = sj;
-  const uint32_t nb = a.nb;
-  const uint32_t p1 = j == UINT_MAX ? 0u : a.ph1[cv.out + j];
-  const uint32_t p2 = j == UINT_MAX ? 0u : a.ph2[cv.out + j];
-  // no positive peak, or a window the search cannot have produced (start past nb, end before
-  // start, wider than kma): no refinement (the neighbourhood must fit the host-sized bins)
-  if (!(gmax > 0.0f) || j == UINT_MAX || p1 >= nb || p2 < p1 || p2 - p1 + 1 > a.kma) {
-    if (tid < (int)nk) { pt[tid].pw = -1.0; pt[tid].j = j == UINT_MAX ? 0u : j; }
-    return;
-  }
-  // neighbourhood: grid window widened by M bins on each side, at most one cycle
-  uint32_t M = a.M;
-  const uint32_t w0 = p2 - p1 + 1;
-  while (M > 0 && w0 + 2 * M > nb) --M;
-  const uint32_t L = w0 + 2 * M;            // coarse bins of the neighbourhood
-  const uint32_t S = a.S;
-  const uint32_t LS = L * S;                // fine bins (host check: <= kMaxFine)
-  const uint32_t E = LS + 1;                // prefix entries per trial
-
-  // ---- scale, reference time, valid count (a non-finite offset leaves no valid sample)
+  // scale, reference time, valid count (a non-finite offset leaves no valid sample)
   const bool off_ok = isfinite(cv.offset);
   float amax = 0.0f, tlo = INFINITY, thi = -INFINITY;
   uint32_t cnt = 0;
-  for (uint32_t i = tid; i < cv.n && off_ok; i += kThreads) {
-    const size_t idx = cv.off + (size_t)i * cv.stride;
-    const float t = a.t[idx], x = a.x[idx];
-    if (valid(t, x)) {
-      amax = fmaxf(amax, fabsf(__fsub_rz(x, cv.offset)));
-      tlo = fminf(tlo, t);
-      thi = fmaxf(thi, t);
-      ++cnt;
+  for (uint32_t i0 = 0; i0 < cv.n; i0 += kHeadThreads * kU) {
+    float tv[kU], xv[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t i = i0 + u * kHeadThreads + tid;
+      const size_t idx = cv.off + (size_t)i * cv.stride;
+      tv[u] = i < cv.n ? __ldg(a.t + idx) : -1.0f;
+      xv[u] = i < cv.n ? __ldg(a.x + idx) : 0.0f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (off_ok && valid(tv[u], xv[u])) {
+        amax = fmaxf(amax, fabsf(__fsub_rz(xv[u], cv.offset)));
+        tlo = fminf(tlo, tv[u]);
+        thi = fmaxf(thi, tv[u]);
+        ++cnt;
+      }
     }
   }
-  amax = block_max(amax, shf);
-  tlo = -block_max(-tlo, shf);
-  thi = block_max(thi, shf);
-  const uint32_t nv = block_sum<unsigned>(cnt, shu);
-  const int sx = amax > 0.0f ? ilogb(kXqMax) - ilogbf(amax) - 1 : 0;
+  float gmax = best;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    tlo = fminf(tlo, __shfl_xor_sync(0xffffffffu, tlo, o));
+    thi = fmaxf(thi, __shfl_xor_sync(0xffffffffu, thi, o));
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  }
+  if (tid == 0) sj = UINT_MAX;
+  if (lane == 0) { shf[0][warp] = gmax; shf[1][warp] = amax; shf[2][warp] = tlo; shf[3][warp] = thi; shn[warp] = cnt; }
+  __syncthreads();
+  gmax = shf[0][0]; amax = shf[1][0]; tlo = shf[2][0]; thi = shf[3][0]; cnt = shn[0];
+  for (int w = 1; w < kW; ++w) {
+    gmax = fmaxf(gmax, shf[0][w]); amax = fmaxf(amax, shf[1][w]);
+    tlo = fminf(tlo, shf[2][w]); thi = fmaxf(thi, shf[3][w]); cnt += shn[w];
+  }
+  if (best == gmax && bj != UINT_MAX) atomicMin(&sj, bj);
+  __syncthreads();
+  if (tid != 0) return;
+  const uint32_t j = sj, nb = a.nb;
+  Head h;
+  h.j = j == UINT_MAX ? 0u : j;
+  h.p1 = j == UINT_MAX ? 0u : a.ph1[cv.out + j];
+  const uint32_t p2 = j == UINT_MAX ? 0u : a.ph2[cv.out + j];
+  // no positive peak, or a window the search cannot have produced (start past nb, end before
+  // start, wider than kma): no refinement (the neighbourhood must fit the host-sized bins)
+  h.ok = gmax > 0.0f && j != UINT_MAX && h.p1 < nb && p2 >= h.p1 && p2 - h.p1 + 1 <= a.kma;
+  // neighbourhood: grid window widened by M bins on each side, at most one cycle
+  uint32_t M = a.M;
+  const uint32_t w0 = p2 - h.p1 + 1;
+  while (M > 0 && w0 + 2 * M > nb) --M;
+  h.M = M;
+  h.L = w0 + 2 * M;
+  h.nv = cnt;
+  h.sx = amax > 0.0f ? ilogb(kXqMax) - ilogbf(amax) - 1 : 0;
   // reference time: the middle of the valid time span, in float32 (order-independent)
-  const float tref = nv ? __fmul_rn(__fadd_rn(tlo, thi), 0.5f) : 0.0f;
+  h.tref = cnt ? __fmul_rn(__fadd_rn(tlo, thi), 0.5f) : 0.0f;
+  a.head[c] = h;
+}
+
+// Shared memory of a trial with L coarse and LS fine bins: exact prefix of the flux and the counts a
+// fine entry, float prefix and row maxima a coarse entry.
+__host__ __device__ inline uint32_t trial_bytes(uint32_t L, uint32_t LS) { return (LS + 1) * 12 + 4 + (L + 1) * 12; }
+
+// |v| in floats, off by less than 2^-23 of itself, without the FP64 pipe's conversion
+__device__ __forceinline__ float ll_mag(long long v) {
+  const int l = (int)(unsigned)(v & 0xffffffffll);
+  const int h = (int)((v - (long long)l) >> 32);
+  return fabsf(__fmaf_rn((float)h, 4294967296.0f, (float)l));
+}
+
+// One block per (curve, group of G consecutive trials): the samples are read and their exact
+// phase pairs formed once for the group, and each trial gets its own fine histogram; a warp then
+// takes a trial at a time.  G is what the neighbourhood leaves room for (wider ones take more
+// shared memory), less where there are too few curves to fill the SMs.  Bound by the phase and
+// histogram work of the samples; the FP64 powers are kept to the windows that FP32 bounds leave
+// (64 curves of 18,000 samples, 65 trials each: 893 -> 303 us, of which the fold takes 200; three
+// trials a block, every block finding peak and scale again, every window twice and 64-bit
+// compare-and-swap atomics before).
+__global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ long long shl[kThreads / 32];
+  const uint32_t c = blockIdx.x;
+  const Head hd = a.head[c];
+  const uint32_t nk_all = 2 * a.K + 1;
+  const uint32_t L = hd.L, S = a.S, LS = L * S;   // coarse and fine bins (host check: LS <= kMaxFine)
+  const uint32_t E = LS + 1;                      // prefix entries per trial
+  uint32_t G = 1;
+  if (hd.ok) {
+    const uint32_t fit = min((uint32_t)kMaxGroup, a.smem / trial_bytes(L, LS));
+    const uint32_t groups = max((nk_all + fit - 1) / fit, a.min_groups);
+    G = (nk_all + groups - 1) / groups;
+  }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  Part *pt = a.part + (size_t)c * nk_all;
+  if (!hd.ok) {
+    if (blockIdx.y == 0)
+      for (uint32_t k = tid; k < nk_all; k += kThreads) { pt[k].pw = -1.0; pt[k].j = hd.j; }
+    return;
+  }
+  const uint32_t k0 = blockIdx.y * G;
+  if (k0 >= nk_all) return;
+  const uint32_t nk = min(G, nk_all - k0);
+  pt += k0;
+  const RefCurve cv = curve_of(a, c);
+  const bool off_ok = isfinite(cv.offset);
+  const uint32_t nb = a.nb, j = hd.j, p1 = hd.p1, M = hd.M;
+  const int sx = hd.sx;
 
   // ---- exact phases: trial k is A + J_k B' - (k - K) R' with B' = frac(t df/K), R' = frac(tref
   // df/K) and J_k = j K + k - K; consecutive trials differ by B' - R'
   const float dfK = ldexpf(cv.df, -a.logK);
-  const unsigned long long Rp = frac64(tref, dfK);
+  const unsigned long long Rp = frac64(hd.tref, dfK);
   const long long J0 = (long long)j * a.K + ((long long)k0 - (long long)a.K);
   const unsigned long long shift0 = (unsigned long long)((long long)k0 - (long long)a.K) * Rp;
   const unsigned long long lo =
       (unsigned long long)((p1 + nb - M) & (nb - 1)) << (64 - a.lognb);  // neighbourhood start
-  long long *hs = reinterpret_cast<long long *>(dyn);                 // [G][E] flux sums
-  int *hc = reinterpret_cast<int *>(hs + (size_t)a.G * E);            // [G][E] counts
-  float *pf = reinterpret_cast<float *>(hc + (size_t)a.G * E);        // [G][E] float prefix
+  // flux sums: two 32-bit words while folding (a 64-bit shared atomic is a loop of
+  // compare-and-swaps), the signed high part of xq = hi 2^20 + lo in the second; exact while a fine
+  // bin holds at most kFineMax samples, checked afterwards
+  long long *hs = reinterpret_cast<long long *>(dyn);                 // [nk][E]
+  int *hc = reinterpret_cast<int *>(hs + (size_t)nk * E);             // [nk][E] counts
+  float2 *cp = reinterpret_cast<float2 *>(hc + (((size_t)nk * E + 1) & ~size_t(1)));   // [nk][L + 1] flux, count
+  float *rm = reinterpret_cast<float *>(cp + (size_t)nk * (L + 1));   // [nk][L + 1] a start's largest bound
   for (uint32_t b = tid; b < nk * E; b += kThreads) { hs[b] = 0; hc[b] = 0; }
   __syncthreads();
-  const double scale = ldexp(1.0, sx);
-  const uint64_t nbS = (uint64_t)a.nb * S;
+  const double unscale = ldexp(1.0, -sx);
+  const uint32_t nbS = a.nb * S;
+  const Scale sc(sx);
   long long stot = 0;
-  for (uint32_t i = tid; i < cv.n && off_ok; i += kThreads) {
-    const size_t idx = cv.off + (size_t)i * cv.stride;
-    const float t = a.t[idx], x = a.x[idx];
-    if (!valid(t, x)) continue;
-    const long long xq = quantise(x, cv.offset, sx);
-    stot += xq;
-    const unsigned long long bp = frac64(t, dfK);
-    unsigned long long ph = frac64(t, cv.fmin) + (unsigned long long)J0 * bp - shift0 - lo;
-    const unsigned long long step = bp - Rp;
-    for (uint32_t g = 0; g < nk; ++g, ph += step) {
-      const uint64_t fb = __umul64hi(ph, nbS);  // fine bin from the neighbourhood start
-      if (fb < LS) {
-        atomicAdd(reinterpret_cast<unsigned long long *>(hs + (size_t)g * E + fb), (unsigned long long)xq);
-        atomicAdd(hc + (size_t)g * E + fb, 1);
+  constexpr int kU = 4;
+  for (uint32_t i0 = 0; i0 < cv.n; i0 += kThreads * kU) {   // kU samples' loads ahead of their uses
+    float tv[kU], xv[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t i = i0 + u * kThreads + tid;
+      const size_t idx = cv.off + (size_t)i * cv.stride;
+      tv[u] = i < cv.n ? __ldg(a.t + idx) : -1.0f;
+      xv[u] = i < cv.n ? __ldg(a.x + idx) : 0.0f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (!off_ok || !valid(tv[u], xv[u])) continue;
+      const long long xq = quantise(xv[u], cv.offset, sc);
+      stot += xq;
+      const unsigned xlo = (unsigned)xq & 0xfffffu, xhi = (unsigned)(xq >> 20);
+      const unsigned long long bp = frac64(tv[u], dfK);
+      unsigned long long ph = frac64(tv[u], cv.fmin) + (unsigned long long)J0 * bp - shift0 - lo;
+      const unsigned long long step = bp - Rp;
+      uint32_t row = 0;
+#pragma unroll 4
+      for (uint32_t g = 0; g < nk; ++g, ph += step, row += E) {
+        // fine bin from the neighbourhood start: floor(ph nb S / 2^64), nb S < 2^20
+        const uint32_t fb = (uint32_t)(((ph >> 32) * nbS + (((ph & 0xffffffffull) * nbS) >> 32)) >> 32);
+        if (fb < LS) {
+          unsigned *h = reinterpret_cast<unsigned *>(hs + row + fb);
+          atomicAdd(h, xlo);
+          atomicAdd(h + 1, xhi);
+          atomicAdd(hc + row + fb, 1);
+        }
       }
     }
   }
   stot = block_sum<long long>(stot, shl);
   __syncthreads();
-  // ---- exclusive prefix sums, one warp per trial: each lane a run of entries, a warp scan of
-  // the runs' totals; the float copy (real flux units) and its largest magnitude for stage 1
-  const uint32_t run = (E + 31) / 32;
-  for (uint32_t g = warp; g < nk; g += kThreads / 32) {
-    long long *H = hs + (size_t)g * E;
-    int *C = hc + (size_t)g * E;
-    const uint32_t b0 = lane * run, b1 = min(E, b0 + run);
-    long long ls = 0;
-    int lc = 0;
-    for (uint32_t b = b0; b < b1; ++b) { ls += H[b]; lc += C[b]; }
-    long long es = ls;
-    int ec = lc;
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long us = __shfl_up_sync(0xffffffffu, es, o);
-      const int uc = __shfl_up_sync(0xffffffffu, ec, o);
-      if (lane >= o) { es += us; ec += uc; }
-    }
-    es -= ls;
-    ec -= lc;
-    float pm = 0.0f;
-    for (uint32_t b = b0; b < b1; ++b) {
-      const long long vs = H[b];
-      const int vc = C[b];
-      H[b] = es;
-      C[b] = ec;
-      const float v = ldexpf(__ll2float_rn(es), -sx);
-      pf[(size_t)g * E + b] = v;
-      pm = fmaxf(pm, fabsf(v));
-      es += vs;
-      ec += vc;
-    }
-    for (int o = 16; o > 0; o >>= 1) pm = fmaxf(pm, __shfl_xor_sync(0xffffffffu, pm, o));
-    if (lane == 0) pmax_s[g] = pm;
-  }
-  __syncthreads();
 
-  // ---- per trial: stage 1, every window of whole bins in the neighbourhood (width in
-  // (kmi, kma] bins), then stage 2, fine edges within one bin of the stage-1 window's edges
-  // (width in (kmi S, kma S] fine bins).  Stage 1 screens in FP32 with error bounds: windows
-  // whose upper bound reaches the largest lower bound are compared exactly in FP64.
+  // ---- a warp per trial from here on: exclusive prefix sums, then stage 1, every window of whole
+  // bins in the neighbourhood (width in (kmi, kma] bins), then stage 2, fine edges within one bin of
+  // the stage-1 window's edges (width in (kmi S, kma S] fine bins).  Both stages screen in FP32 with
+  // error bounds: windows whose upper bound reaches a lower bound of the largest power are compared
+  // exactly in FP64.
   const double N = (double)cv.ntrue;
   const float Nf = (float)cv.ntrue;
   const int kkmi = (int)(cv.kkmi < 5u ? 5u : cv.kkmi);
-  const uint32_t kmaL = a.kma < L ? a.kma : L;
-  const uint32_t nw1 = L * kmaL;
-  __shared__ double wp[kThreads / 32];
-  __shared__ uint32_t wa[kThreads / 32], wb[kThreads / 32];
-  auto block_best = [&](double &bp, uint32_t &ba, uint32_t &bb) {  // fixed-order argmax
-    for (int o = 16; o > 0; o >>= 1) {
-      const double op = __shfl_xor_sync(0xffffffffu, bp, o);
-      const uint32_t oa = __shfl_xor_sync(0xffffffffu, ba, o);
-      const uint32_t ob = __shfl_xor_sync(0xffffffffu, bb, o);
-      if (better(op, oa, ob, bp, ba, bb)) { bp = op; ba = oa; bb = ob; }
-    }
-    __syncthreads();
-    if (lane == 0) { wp[warp] = bp; wa[warp] = ba; wb[warp] = bb; }
-    __syncthreads();
-    bp = wp[0]; ba = wa[0]; bb = wb[0];
-    for (int w = 1; w < kThreads / 32; ++w)
-      if (better(wp[w], wa[w], wb[w], bp, ba, bb)) { bp = wp[w]; ba = wa[w]; bb = wb[w]; }
+  const float kkmi_f = (float)kkmi;
+  const int kma = (int)a.kma, kmi = (int)a.kmi, iL = (int)L;
+  auto warp_max = [](float v) {   // non-negative values
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
   };
-  for (uint32_t g = 0; g < nk; ++g) {
-    const long long *H = hs + (size_t)g * E;
-    const int *C = hc + (size_t)g * E;
-    const float *P = pf + (size_t)g * E;
+  for (uint32_t g = warp; g < nk; g += kThreads / 32) {
+    long long *H = hs + (size_t)g * E;
+    int *C = hc + (size_t)g * E;
+    float2 *P = cp + (size_t)g * (L + 1);
+    float *R = rm + (size_t)g * (L + 1);
+    {
+      // each lane a run of entries (an odd number: fewer bank conflicts), a warp scan of the totals
+      const uint32_t run = ((E + 31) / 32) | 1u;
+      const uint32_t b0 = min(E, lane * run), b1 = min(E, b0 + run);
+      long long ls = 0;
+      int lc = 0, cmax = 0;
+      for (uint32_t b = b0; b < b1; ++b) {
+        const uint2 v = reinterpret_cast<const uint2 *>(H)[b];
+        H[b] = ((long long)(int)v.y << 20) + (long long)v.x;
+        ls += H[b];
+        lc += C[b];
+        cmax = max(cmax, C[b]);
+      }
+      if (__any_sync(0xffffffffu, cmax > kFineMax)) {   // rare: this trial's sums again, 64 bits at a time
+        for (uint32_t b = lane; b < E; b += 32) H[b] = 0;
+        __syncwarp();
+        for (uint32_t i = lane; i < cv.n; i += 32) {
+          const size_t idx = cv.off + (size_t)i * cv.stride;
+          const float t = a.t[idx], x = a.x[idx];
+          if (!off_ok || !valid(t, x)) continue;
+          const unsigned long long bp = frac64(t, dfK);
+          const unsigned long long ph = frac64(t, cv.fmin) + (unsigned long long)J0 * bp - shift0 - lo + g * (bp - Rp);
+          const uint64_t fb = __umul64hi(ph, (uint64_t)nbS);
+          if (fb < LS)
+            atomicAdd(reinterpret_cast<unsigned long long *>(H + fb), (unsigned long long)quantise(x, cv.offset, sc));
+        }
+        __syncwarp();
+        ls = 0;
+        for (uint32_t b = b0; b < b1; ++b) ls += H[b];
+      }
+      long long es = ls;
+      int ec = lc;
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long us = __shfl_up_sync(0xffffffffu, es, o);
+        const int uc = __shfl_up_sync(0xffffffffu, ec, o);
+        if (lane >= o) { es += us; ec += uc; }
+      }
+      es -= ls;
+      ec -= lc;
+      for (uint32_t b = b0; b < b1; ++b) {
+        const long long vs = H[b];
+        const int vc = C[b];
+        H[b] = es;
+        C[b] = ec;
+        es += vs;
+        ec += vc;
+      }
+    }
+    __syncwarp();
+    // the coarse entries as floats (real flux units) and their largest magnitude
+    float pm = 0.0f;
+    for (int e = lane; e <= iL; e += 32) {
+      const float v = ldexpf(__ll2float_rn(H[e * S]), -sx);
+      P[e] = make_float2(v, (float)C[e * S]);
+      pm = fmaxf(pm, fabsf(v));
+    }
+    pm = warp_max(pm);
+    __syncwarp();
     // |P - exact| <= 2^-24 |exact| per entry, so a difference is off by at most 2^-23 pmax
     // plus 2^-24 of itself (both taken twice here); den is exact to 2^-24 and the quotient
     // from __fdividef within 2 ulp, inside the 2^-20 factors
-    const float e0 = ldexpf(pmax_s[g], -22);
-    auto power = [&](uint32_t ws, uint32_t we, double &pw) -> bool {
+    const float e0 = ldexpf(pm, -22);
+    auto power = [&](int ws, int we, double &pw) -> bool {
       const int kk = C[we] - C[ws];
       if (kk <= kkmi) return false;
       const double den = (double)kk * (N - (double)kk);
       if (!(den > 0.0)) return false;
-      const double sv = (double)(H[we] - H[ws]) / scale;
+      const double sv = (double)(H[we] - H[ws]) * unscale;
       pw = sv * sv / den;
       return true;
     };
-    auto bounds = [&](uint32_t ws, uint32_t we, float &plo, float &phi) -> bool {
-      const int kk = C[we] - C[ws];
-      if (kk <= kkmi) return false;
-      const float den = (float)kk * (Nf - (float)kk);
-      if (!(den > 0.0f)) return false;
-      const float sv = fabsf(P[we] - P[ws]);
-      const float err = e0 + ldexpf(sv, -22);
-      const float lo_ = fmaxf(sv - err, 0.0f), hi_ = sv + err;
-      plo = __fdividef(lo_ * lo_, den) * (1.0f - 1.0f / 1048576.0f);
-      phi = __fdividef(hi_ * hi_, den) * (1.0f + 1.0f / 1048576.0f);
-      return true;
+    auto upper = [&](float2 A, float2 B) -> float {   // 0 where the window does not count
+      const float kk = B.y - A.y, den = kk * (Nf - kk);
+      const float sv = fabsf(B.x - A.x), hi = sv + (e0 + sv * (1.0f / 4194304.0f));
+      return kk > kkmi_f && den > 0.0f ? __fdividef(hi * hi, den) * (1.0f + 1.0f / 1048576.0f) : 0.0f;
     };
     // (a float prefix near the underflow range would break the bounds: no screening there)
     float thr = 0.0f;
-    for (uint32_t q = tid; q < nw1 && sx < 100; q += kThreads) {
-      const uint32_t ac = q / kmaL, w = q - ac * kmaL + 1;
-      if (w <= a.kmi || ac + w > L) continue;
-      float plo, phi;
-      if (bounds(ac * S, (ac + w) * S, plo, phi)) thr = fmaxf(thr, plo);
+    if (sx < 100) {
+      float top = 0.0f, lower = 0.0f;
+      for (int s = 0; s < iL; ++s) {
+        const float2 A = P[s];
+        const int wmax = min(kma, iL - s);
+        float rowmax = 0.0f;
+        for (int w = kmi + 1 + lane; w <= wmax; w += 32) {
+          const float2 B = P[s + w];
+          const float phi = upper(A, B);
+          rowmax = fmaxf(rowmax, phi);
+          if (phi > top) {   // the lane's best bound so far: the lower bound of its window
+            top = phi;
+            const float kk = B.y - A.y, den = kk * (Nf - kk);
+            const float sv = fabsf(B.x - A.x), low = fmaxf(sv - (e0 + sv * (1.0f / 4194304.0f)), 0.0f);
+            lower = fmaxf(lower, __fdividef(low * low, den) * (1.0f - 1.0f / 1048576.0f));
+          }
+        }
+        rowmax = warp_max(rowmax);
+        if (lane == 0) R[s] = rowmax;
+      }
+      thr = warp_max(lower);
     }
-    thr = block_max(thr, shf);
+    __syncwarp();
     double bp = -1.0;
     uint32_t ba = UINT_MAX, bb = UINT_MAX;
-    for (uint32_t q = tid; q < nw1; q += kThreads) {
-      const uint32_t ac = q / kmaL, w = q - ac * kmaL + 1;
-      if (w <= a.kmi || ac + w > L) continue;
-      float plo, phi;
-      if (!bounds(ac * S, (ac + w) * S, plo, phi) || phi < thr) continue;
-      double pw;
-      if (power(ac * S, (ac + w) * S, pw) && better(pw, ac * S, (ac + w) * S, bp, ba, bb)) {
-        bp = pw; ba = ac * S; bb = (ac + w) * S;
+    auto warp_best = [&]() {   // fixed-order argmax
+      for (int o = 16; o > 0; o >>= 1) {
+        const double op = __shfl_xor_sync(0xffffffffu, bp, o);
+        const uint32_t oa = __shfl_xor_sync(0xffffffffu, ba, o);
+        const uint32_t ob = __shfl_xor_sync(0xffffffffu, bb, o);
+        if (better(op, oa, ob, bp, ba, bb)) { bp = op; ba = oa; bb = ob; }
+      }
+    };
+    for (int s0 = 0; s0 < iL; s0 += 32) {
+      const bool in = s0 + lane < iL && (sx >= 100 || R[s0 + lane] >= thr);
+      for (unsigned rows = __ballot_sync(0xffffffffu, in); rows; rows &= rows - 1) {
+        const int s = s0 + __ffs(rows) - 1;
+        const float2 A = P[s];
+        const int wmax = min(kma, iL - s);
+        for (int w = kmi + 1 + lane; w <= wmax; w += 32) {
+          if (sx < 100 && upper(A, P[s + w]) < thr) continue;
+          const uint32_t ws = s * S, we = (s + w) * S;
+          double pw;
+          if (power((int)ws, (int)we, pw) && better(pw, ws, we, bp, ba, bb)) { bp = pw; ba = ws; bb = we; }
+        }
       }
     }
-    block_best(bp, ba, bb);
+    warp_best();
     if (ba != UINT_MAX) {
       const uint32_t a0 = ba > S ? ba - S : 0u, a1 = ba + S < LS ? ba + S : LS;
       const uint32_t b0 = bb > S ? bb - S : 0u, b1 = bb + S < LS ? bb + S : LS;
       const uint32_t na = a1 - a0 + 1, nbw = b1 - b0 + 1;
       const uint32_t wmin = a.kmi * S, wmax = a.kma * S;
-      for (uint32_t q = tid; q < na * nbw; q += kThreads) {
-        const uint32_t ws = a0 + q / nbw, we = b0 + (q - (q / nbw) * nbw);
+      // the power in quantised units, within 2^-20 of itself (0 where the window does not count)
+      auto approx = [&](uint32_t ws, uint32_t we) -> float {
+        if (we <= ws || we - ws <= wmin || we - ws > wmax) return 0.0f;
+        const float kk = (float)(C[we] - C[ws]), den = kk * (Nf - kk);
+        const float sv = ll_mag(H[we] - H[ws]);
+        return kk > kkmi_f && den > 0.0f ? __fdividef(sv * sv, den) : 0.0f;
+      };
+      float top = 0.0f;
+      for (uint32_t q = lane; q < na * nbw; q += 32) top = fmaxf(top, approx(a0 + q / nbw, b0 + q % nbw));
+      const float low = warp_max(top) * (1.0f - 1.0f / 262144.0f);
+      for (uint32_t q = lane; q < na * nbw; q += 32) {
+        const uint32_t ws = a0 + q / nbw, we = b0 + q % nbw;
         if (we <= ws || we - ws <= wmin || we - ws > wmax) continue;
+        if (approx(ws, we) < low) continue;
         double pw;
-        if (power(ws, we, pw) && better(pw, ws, we, bp, ba, bb)) { bp = pw; ba = ws; bb = we; }
+        if (power((int)ws, (int)we, pw) && better(pw, ws, we, bp, ba, bb)) { bp = pw; ba = ws; bb = we; }
       }
-      block_best(bp, ba, bb);
+      warp_best();
     }
-    if (tid == 0) {
+    if (lane == 0) {
       Part &o = pt[g];
       o.pw = ba == UINT_MAX ? -1.0 : bp;
       o.s = ba == UINT_MAX ? 0 : H[bb] - H[ba];
@@ -369,11 +512,11 @@ __global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a)
       o.a = ba;
       o.b = bb;
       o.stot = stot;
-      o.nv = nv;
+      o.nv = hd.nv;
       o.j = j;
       o.p1 = (p1 + nb - M) & (nb - 1);  // neighbourhood start bin
       o.sx = sx;
-      o.tref = tref;
+      o.tref = hd.tref;
     }
   }
 }
@@ -451,23 +594,29 @@ int refine_common(RefArgs &a, uint32_t count, void *workspace, size_t workspace_
   if ((uint64_t)(a.kma + 2 * a.M) * a.S > (uint64_t)kMaxFine)
     return fail(GTRAP_ERR_INVALID_ARG, "%s: (kma + 2M) * S = %u exceeds %d fine bins", name,
                 (a.kma + 2 * a.M) * a.S, kMaxFine);
-  const size_t need = (size_t)count * (2 * a.K + 1) * sizeof(Part);
+  const size_t parts = gtrap::align256((size_t)count * (2 * (size_t)a.K + 1) * sizeof(Part));
+  const size_t need = parts + (size_t)count * sizeof(Head);
   if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < need)
     return fail(GTRAP_ERR_WORKSPACE, "%s: workspace of %zu bytes (256-byte aligned) needed", name, need);
   if (count > 65535u * 4u) return fail(GTRAP_ERR_INVALID_ARG, "%s: at most %u curves per call", name, 65535u * 4u);
   a.lognb = gtrap::ilog2u(a.nb);
   a.logK = gtrap::ilog2u(a.K);
   a.part = reinterpret_cast<Part *>(workspace);
-  // trials per block: as many fine histograms (16 bytes an entry) as fit the block's budget
-  const size_t per_trial = (size_t)((a.kma + 2 * a.M) * a.S + 1) * 16;
-  uint32_t G = (uint32_t)(kSmemBudget / per_trial);
-  if (G < 1) G = 1;
-  if (G > (uint32_t)kMaxGroup) G = kMaxGroup;
-  if (G > 2 * a.K + 1) G = 2 * a.K + 1;
-  a.G = G;
-  const size_t smem = (size_t)G * per_trial;
+  a.head = reinterpret_cast<Head *>((char *)workspace + parts);
+  // trials per block: chosen on the device by the neighbourhood's size, within a block's budget; two
+  // blocks an SM's worth of groups where there are few curves
+  const uint32_t nk = 2 * a.K + 1, widest = a.kma + 2 * a.M;
+  const size_t worst = trial_bytes(widest, widest * a.S);
+  const size_t smem = worst > kSmemBudget ? worst : kSmemBudget;
+  a.smem = (uint32_t)smem;
+  const uint32_t want = ((uint32_t)gtrap::sm_count() * 2 + count - 1) / count;
+  a.min_groups = want > nk ? nk : want;
+  uint32_t fit = (uint32_t)(smem / worst);
+  if (fit > (uint32_t)kMaxGroup) fit = kMaxGroup;
+  const uint32_t groups = (nk + fit - 1) / fit > a.min_groups ? (nk + fit - 1) / fit : a.min_groups;
   GTRAP_TRY(gtrap::ensure_smem((const void *)refine_trial_kernel, smem, name));
-  const uint32_t groups = (2 * a.K + 1 + G - 1) / G;
+  refine_head_kernel<<<count, kHeadThreads, 0, stream>>>(a);
+  GTRAP_TRY(gtrap::check_launch("refine_head_kernel"));
   refine_trial_kernel<<<dim3(count, groups), kThreads, smem, stream>>>(a);
   GTRAP_TRY(gtrap::check_launch("refine_trial_kernel"));
   refine_pick_kernel<<<(count + 3) / 4, 128, 0, stream>>>(a, count);
@@ -479,7 +628,8 @@ int refine_common(RefArgs &a, uint32_t count, void *workspace, size_t workspace_
 extern "C" {
 
 size_t gtrap_bls_refine_workspace_size(uint32_t ncurves, uint32_t K) {
-  return gtrap::align256((size_t)ncurves * (2 * (size_t)K + 1) * sizeof(Part)) + 256;
+  return gtrap::align256((size_t)ncurves * (2 * (size_t)K + 1) * sizeof(Part)) +
+         gtrap::align256((size_t)ncurves * sizeof(Head)) + 256;
 }
 
 int gtrap_bls_refine(const float *blsp, const uint32_t *phase1, const uint32_t *phase2, const float *lc,

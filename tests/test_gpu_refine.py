@@ -193,3 +193,25 @@ def test_refine_degenerate_curves(cuda):
         o = OR.refine_curve(t[:, 2], lc[:, 2], off[2], ntrue[2], sr[2], p1[2], p2[2], g["fmin"], g["df"],
                             1024, 103, 5, 10, K=KR, S=SR_, M=MR)
         _check(recs[2], o)
+
+
+@pytest.mark.parametrize("n,period", [(30000, 0.25), (300, 0.25), (9000, 0.02)])
+def test_refine_crowded_fine_bins(cuda, n, period):
+    """Times that fall on a few phases: fine bins of thousands of samples (the two 32-bit words of a
+    sum hold 2047, the trial is then folded again in 64 bits), of a few, and a single one; a lone curve
+    (one trial a block) and the same curve among many (several trials a block) give the same bits."""
+    rng = np.random.default_rng(n)
+    cad = np.float32(period / 8)
+    t = (np.arange(n) * cad).astype(np.float32)
+    x = rng.normal(0.0, 1e-3, n).astype(np.float32)
+    x[::8] -= 2e-3
+    nf, fmin, df = 40, np.float32(0.9 / period), np.float32(0.2 / period / 40)
+    g = dict(nf=nf, nb=256, kma=26, kmi=1, kkmi=5, fmin=float(fmin), df=float(df))
+    off, ntrue = np.zeros(1, np.float32), np.full(1, n, np.uint32)
+    sr, p1, p2, recs = _search_and_refine(x[:, None], t[:, None], ntrue, off, g, cuda)
+    o = OR.refine_curve(t, x, off[0], n, sr[0], p1[0], p2[0], g["fmin"], g["df"], g["nb"], g["kma"], g["kmi"], g["kkmi"],
+                        K=KR, S=SR_, M=MR)
+    _check(recs[0], o)
+    many = np.tile(x[:, None], (1, 200)), np.tile(t[:, None], (1, 200))
+    _, _, _, recs2 = _search_and_refine(*many, np.repeat(ntrue, 200), np.repeat(off, 200), g, cuda)
+    assert all(r.tobytes() == recs[0].tobytes() for r in recs2)
