@@ -32,10 +32,16 @@ def _d64(a, dev):
 
 def _sorted_series(t, x, dev):
     """Finite-time samples sorted by time (a non-finite time lies in no region)."""
-    t = _d64(t, dev)
+    th = np.asarray(t, dtype=np.float64).reshape(-1)
+    # a curve as it was observed, sorted and complete, needs neither the selection nor the sort on the
+    # device (some 25 launches and two waits: 0.4 ms for 18,000 samples, the look 0.02 ms)
+    ordered = th.size == 0 or bool(np.isfinite(th[0]) and np.isfinite(th[-1]) and (th[1:] >= th[:-1]).all())
+    t = _d64(th, dev)
     x = _d64(x, dev)
     if t.numel() != x.numel():
         raise ValueError("t and x must have the same length")
+    if ordered:
+        return t, x
     keep = torch.isfinite(t)
     t, x = t[keep], x[keep]
     order = torch.argsort(t, stable=True)

@@ -106,3 +106,54 @@ def test_tlsfit_reference_golden(cuda):
         assert (W, L, T0) == (bW, bL, bT0), k
         assert H == pytest.approx(bH, rel=1e-9) and off == pytest.approx(boff, rel=1e-12)
         np.testing.assert_allclose(xpre, g["xpre_%d" % k], rtol=1e-9, atol=1e-12)
+
+
+def test_infinite_flux_and_empty_windows(cuda):
+    """Fluxes of +-inf and NaN beside the finite ones, a template whose window holds none but NaN, an
+    epoch on a sample (tn = 0 times an infinite flux), sorted times (no sort on the device) and the
+    same curve shuffled."""
+    t, x = _curve(9, nan_t=0.0, shuffle=False)
+    x[[100, 700]] = np.inf
+    x[900] = -np.inf
+    x[300:340] = np.nan
+    Wl, Ll = np.array([0.2, 0.6]), np.array([0.05, 0.3])
+    tl = np.array([t[100], t[320], t[320] + 0.2, t[900], 12.3, 15.0])
+    got = [a.cpu().numpy() for a in tls.chi2_grid(t, x, Wl, Ll, tl)]
+    p = np.random.default_rng(3).permutation(t.size)
+    for a, b in zip(got, tls.chi2_grid(t[p], x[p], Wl, Ll, tl)):
+        np.testing.assert_array_equal(a, b.cpu().numpy())
+    k = 0
+    for W in Wl:
+        for L in Ll:
+            for T in tl:
+                with np.errstate(all="ignore"):
+                    H, res, n, xs = tls_cpu.get_chi2Hmax(t, x, W, L, T)
+                np.testing.assert_allclose([got[0][k], got[1][k], got[3][k]], [H, res, xs], rtol=1e-9, atol=1e-12)
+                assert got[2][k] == n
+                k += 1
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 65536, 65537, 200001])
+def test_nanargmax_over_its_blocks(cuda, n):
+    import torch
+    from gtrap_gb300 import _native as N
+    from gtrap_gb300._dev import as_ptr
+    rng = np.random.default_rng(n)
+    idx = torch.empty(1, dtype=torch.int64, device=cuda)
+
+    def run(v):
+        d = torch.from_numpy(v).to(cuda)
+        N.call("gtrap_nanargmax", as_ptr(d), v.size, as_ptr(idx), torch.cuda.current_stream().cuda_stream)
+        return int(idx.item())
+
+    v = rng.normal(size=n)
+    assert run(v) == np.argmax(v)
+    ties = np.round(v)
+    ties[rng.random(n) < 0.3] = -0.0
+    assert run(ties) == np.argmax(ties)
+    ties[rng.random(n) < 0.5] = np.nan
+    if not np.isnan(ties).all():
+        assert run(ties) == np.nanargmax(ties)
+    assert run(-np.abs(v)) == np.argmax(-np.abs(v))
+    assert run(np.full(n, -np.inf)) == 0
+    assert run(np.full(n, np.nan)) == -1
