@@ -69,6 +69,10 @@ int gfilter_groups_image(const float *in, float *out, uint32_t n, uint32_t nq, u
 int gfilter_groups_columns(const float *in, float *out, uint32_t n, uint32_t nq, uint32_t r, cudaStream_t stream);
 int gfilter_groups_packed(const float *in, float *out, const unsigned long long *off, const uint32_t *n,
                           uint32_t ncurves, uint32_t max_n, uint32_t r, cudaStream_t stream);
+// Larger radii: sorted cores in shared memory (columns: lens or under 12 curves), as far as they fit.
+size_t gfilter_merge_smem(uint32_t r);
+int gfilter_merge(const float *in, float *out, const unsigned long long *off, const uint32_t *lens, uint32_t ncurves,
+                  uint32_t n, uint32_t r, cudaStream_t stream);
 
 // frac(t*f) * 2^64 for float32 t and f, exact whenever the product is >= 2^-17.
 __device__ __forceinline__ uint64_t frac64(float t, float f) {

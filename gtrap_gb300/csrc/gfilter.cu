@@ -15,6 +15,9 @@
 // curves of 3.5 M samples 462 / 47 us, one of 19,254 69 / 10 us; r = 5 119 / 47, r = 63 2421 / 153
 // us on 65,536 x 128.
 //
+// Radii of 64 and more, as far as their cores fit in shared memory (r <= 888 with 227 KB): groups of
+// 16 rows whose common core is kept sorted in shared memory and moves by merging (gfilter_merge.cu).
+//
 // Other radii: every warp owns 32 adjacent curves (one per lane, so each row it touches is one
 // coalesced 128-byte line of the [n, nq] image) and a run of consecutive rows.  Each lane keeps
 // its window sorted in shared memory, laid out [rank][lane] so that every access is
@@ -187,6 +190,8 @@ int gtrap_gfilter(const float *in, float *out, uint32_t n, uint32_t nq, uint32_t
   if (n > 0x7fffffffu || nq > 0x7fffffffu)
     return fail(GTRAP_ERR_INVALID_ARG, "gfilter: n and nq must be below 2^31");
   if (r >= kGroupMinR && r <= kGroupMaxR) return gfilter_groups_image(in, out, n, nq, r, stream);
+  if (r > kGroupMaxR && gfilter_merge_smem(r) <= (size_t)max_smem_optin())
+    return gfilter_merge(in, out, nullptr, nullptr, nq, n, r, stream);
   const size_t w = 2 * (size_t)r + 1;
   const size_t per_warp = w * 32 * sizeof(float);
   const size_t budget = (size_t)max_smem_optin();
@@ -225,6 +230,8 @@ int gtrap_gfilter_packed(const float *in, float *out, const uint64_t *off, const
   if (in == out) return fail(GTRAP_ERR_INVALID_ARG, "gfilter_packed: in and out must not alias");
   if (r >= kGroupMinR && r <= kGroupMaxR)
     return gfilter_groups_packed(in, out, (const unsigned long long *)off, n, ncurves, max_n, r, stream);
+  if (r > kGroupMaxR && gfilter_merge_smem(r) <= (size_t)max_smem_optin())
+    return gfilter_merge(in, out, (const unsigned long long *)off, n, ncurves, max_n, r, stream);
   const size_t w = 2 * (size_t)r + 1;
   const size_t per_warp = w * 32 * sizeof(float);
   const size_t budget = (size_t)max_smem_optin();

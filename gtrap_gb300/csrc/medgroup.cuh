@@ -17,15 +17,22 @@
 
 namespace gtrap {
 
-__device__ __forceinline__ void cx(float &a, float &b) {
-  const float lo = fminf(a, b), hi = fmaxf(a, b);
+// The networks sort floats, or integer keys of the same order.
+__device__ __forceinline__ float lesser(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float greater(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ int lesser(int a, int b) { return min(a, b); }
+__device__ __forceinline__ int greater(int a, int b) { return max(a, b); }
+
+template <class V>
+__device__ __forceinline__ void cx(V &a, V &b) {
+  const V lo = lesser(a, b), hi = greater(a, b);
   a = lo;
   b = hi;
 }
 
 // Batcher's odd-even merge sort of v[0 .. N), N a power of two.
-template <int N>
-__device__ __forceinline__ void net_sort(float (&v)[N]) {
+template <int N, class V>
+__device__ __forceinline__ void net_sort(V (&v)[N]) {
 #pragma unroll
   for (int p = 1; p < N; p *= 2) {
 #pragma unroll
@@ -41,8 +48,8 @@ __device__ __forceinline__ void net_sort(float (&v)[N]) {
 }
 
 // A bitonic sequence into ascending order.
-template <int N>
-__device__ __forceinline__ void net_clean(float (&v)[N]) {
+template <int N, class V>
+__device__ __forceinline__ void net_clean(V (&v)[N]) {
 #pragma unroll
   for (int s = N / 2; s >= 1; s /= 2) {
 #pragma unroll
@@ -65,14 +72,14 @@ __device__ __forceinline__ void net_merge(const float (&a)[N], const float (&b)[
 // The middle H of the 3H values of a (2H, ascending) and b (H, ascending), ascending: the H
 // smallest are among a's lower half and b, the H largest of the rest among what is left of those
 // and a's upper half.
-template <int H>
-__device__ __forceinline__ void net_middle(const float (&a)[2 * H], const float (&b)[H], float (&out)[H]) {
-  float x[H];
+template <int H, class V>
+__device__ __forceinline__ void net_middle(const V (&a)[2 * H], const V (&b)[H], V (&out)[H]) {
+  V x[H];
 #pragma unroll
-  for (int i = 0; i < H; ++i) x[i] = fmaxf(a[i], b[H - 1 - i]);
+  for (int i = 0; i < H; ++i) x[i] = greater(a[i], b[H - 1 - i]);
   net_clean(x);
 #pragma unroll
-  for (int i = 0; i < H; ++i) out[i] = fminf(x[i], a[2 * H - 1 - i]);
+  for (int i = 0; i < H; ++i) out[i] = lesser(x[i], a[2 * H - 1 - i]);
   net_clean(out);
 }
 
@@ -104,14 +111,14 @@ __device__ __forceinline__ void net_middle_of_two(const float (&a)[N], const flo
 // The medians of windows K0 .. K0 + T - 1 of a group of T0 from the T middle values of their
 // common core.  left[j] (j = 1 .. T0 - 1): the row that windows 0 .. j - 1 hold; right[j]
 // (j = 0 .. T0 - 2): the row that windows j + 1 .. T0 - 1 hold.
-template <int T0, int T, int K0>
-__device__ __forceinline__ void median_halves(const float (&core)[T], const float (&left)[T0],
-                                              const float (&right)[T0], float (&med)[T0]) {
+template <int T0, int T, int K0, class V>
+__device__ __forceinline__ void median_halves(const V (&core)[T], const V (&left)[T0], const V (&right)[T0],
+                                              V (&med)[T0]) {
   if constexpr (T == 1) {
     med[K0] = core[0];
   } else {
     constexpr int H = T / 2;
-    float e[H], mid[H];
+    V e[H], mid[H];
 #pragma unroll
     for (int i = 0; i < H; ++i) e[i] = left[K0 + H + i];
     net_sort(e);

@@ -150,3 +150,34 @@ def test_gfilter_groups_at_their_edges(cuda, n, r):
         np.testing.assert_array_equal(got, want[:, cols])
     for q, got in enumerate(_packed(cuda, [x[:, q].copy() for q in range(5)] + [x[:n // 2 + 1, 5].copy()], r)[:5]):
         np.testing.assert_array_equal(got, want[:, q])
+
+
+@pytest.mark.parametrize("n,r", [(1, 64), (17, 71), (130, 72), (700, 65), (700, 128), (2065, 100), (2065, 128),
+                                 (5000, 300), (1500, 888), (1500, 900)])
+def test_gfilter_merged_cores(cuda, n, r):
+    """Radii past the grouped medians (cores that move by merging, and at the largest the
+    sliding windows), with cores of every remainder of 16, runs of one and of several groups, series
+    shorter and longer than a window, ties, equal series and infinities: image (one, three and 40
+    curves) and packed, equal to medfilt."""
+    rng = np.random.default_rng(64 * n + r)
+    x = rng.normal(1.0, 1e-3, size=(n, 40)).astype(np.float32)
+    x[:, 1] = rng.integers(-1, 2, n)
+    x[:, 2] = 0.5
+    x[:, 3] = np.sin(np.arange(n) / 50.0)
+    x[rng.random((n, 40)) < 0.002] = np.inf
+    x[rng.random((n, 40)) < 0.002] = -np.inf
+    want = oracle.medfilt_residual(x, r)
+    for cols in (slice(0, 1), slice(0, 3), slice(0, 40)):
+        got = api.gfilter(torch.from_numpy(np.ascontiguousarray(x[:, cols])).to(cuda), r).cpu().numpy()
+        np.testing.assert_array_equal(got, want[:, cols])
+    for q, got in enumerate(_packed(cuda, [x[:, q].copy() for q in range(5)] + [x[:n // 2 + 1, 5].copy()], r)[:5]):
+        np.testing.assert_array_equal(got, want[:, q])
+
+
+def test_gfilter_merged_cores_long_runs(cuda):
+    """Runs of many groups (both directions of the pass) and a last run cut short."""
+    rng = np.random.default_rng(9)
+    x = rng.normal(1.0, 1e-3, size=(6001, 1500)).astype(np.float32)
+    got = api.gfilter(torch.from_numpy(x).to(cuda), 200).cpu().numpy()
+    cols = [0, 31, 32, 777, 1499]
+    np.testing.assert_array_equal(got[:, cols], oracle.medfilt_residual(np.ascontiguousarray(x[:, cols]), 200))
