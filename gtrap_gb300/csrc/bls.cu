@@ -1118,6 +1118,15 @@ size_t ws_size(uint32_t n, uint32_t nq, uint32_t flags, bool full) {
   return s + 256;
 }
 
+// Frequencies per block of a launch whose blocks of the usual size would fill the SMs less than twice (a
+// lone curve): smaller blocks leave fewer SMs idle in the last wave, or at all.  Before / now, one
+// curve, two blocks an SM: 10,000 samples, 2048 frequencies, nb = 2048 (342 blocks of 6 / 512 of 4)
+// 152 / 142 us; 1000 frequencies (167 / 250) 110 / 97 us; 65,536 samples, 2048 frequencies 430 / 363 us;
+// 18,000 samples, 4096 frequencies, nb = 1024 (512 of 8 / 1024 of 4) 294 / 267 us.  From 2 waves of
+// blocks on the usual size is as fast (4096 frequencies, nb = 2048: 223 / 223 us) or faster (8192:
+// 526 / 536 us).  Blocks of 2 or 3 re-read the samples too often (149 and 143 us in the first case).
+constexpr uint32_t kFewF = 4;
+
 int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const float *lc,
             const float *tu, const float *offset, const uint32_t *ntrue, uint32_t n, uint32_t nq,
             uint32_t nf, uint32_t nb, uint32_t kma, uint32_t kmi, uint32_t kkmi, float fmin,
@@ -1179,6 +1188,8 @@ int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const fl
 
   Plan p;
   GTRAP_TRY(make_plan(nb, kma, nf, 0, &p));
+  if (p.F > kFewF && kFewF % p.G == 0 && (uint64_t)p.tiles * nq <= 2ull * kMinBlocks * gtrap::sm_count())
+    GTRAP_TRY(make_plan(nb, kma, nf, kFewF, &p));
   const BlsShape sh = shape_of(p, nb, kma, kmi_eff, kkmi_eff, flags);
   BlsArgs ba;
   ba.blsp = blsp; ba.ph1 = phase1; ba.ph2 = phase2;

@@ -169,3 +169,21 @@ def test_scan_chunks_at_their_edges(cuda, n, nb, kma, kmi):
     osr, op1, op2, opmax = oracle.bls(wl.lc, wl.tu, wl.nf, nb, kma, kmi, 1, wl.fmin, wl.df)
     _check_spectrum(sr.cpu().numpy(), p1.cpu().numpy(), p2.cpu().numpy(), osr, op1, op2, opmax,
                     wl.lc, wl.tu, dict(nb=nb, fmin=wl.fmin, df=wl.df))
+
+
+@pytest.mark.parametrize("nf,nb", [(3, 2048), (1000, 2048), (3644, 2048), (3654, 2048), (4100, 1024), (700, 1000)])
+def test_lone_curve_takes_smaller_blocks(cuda, nf, nb):
+    """A launch of few blocks takes fewer frequencies a block: the same bits as the curve gets in a
+    batch that fills the GPU, at both ends of the rule."""
+    rng = np.random.default_rng(nf + nb)
+    n, nq = 1500, 40
+    tu = torch.from_numpy(np.sort(rng.uniform(0, 60, (n, 1)), axis=0).astype(np.float32)).to(cuda)
+    lc = torch.from_numpy(rng.normal(0, 1e-3, (n, 1)).astype(np.float32)).to(cuda)
+    kw = dict(nf=nf, nb=nb, kma=nb // 10, kmi=nb // 200, kkmi=8, fmin=0.05, df=2.0 / nf)
+
+    def run(k):
+        return api.geebls(lc.expand(n, k).contiguous(), tu.expand(n, k).contiguous(), torch.zeros(k, device=cuda),
+                          torch.full((k,), n, dtype=torch.int32, device=cuda), **kw)
+    for one, many in zip(run(1), run(nq)):
+        assert torch.equal(one[0].view(torch.int32), many[0].view(torch.int32))
+        assert torch.equal(one[0].view(torch.int32), many[-1].view(torch.int32))
