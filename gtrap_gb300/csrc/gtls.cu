@@ -45,6 +45,14 @@ constexpr int kWarps = 8;
 constexpr int kTlsThreads = kWarps * 32;
 constexpr int kTE = 64;          // epochs per tile
 constexpr int kHalves = kTE / 32;
+// A launch whose half tiles make at most this many halves of a wave of resident blocks takes each tile as two
+// blocks of half its epochs: a tile's time is its staging and the chain of its warps' (half, width)
+// units, so half tiles shorten the chain where SMs would otherwise hold few blocks; past that the
+// second staging costs more.  Before / now, 8 widths from 0.5 to 8 h, 2-min cadence, one
+// curve (launches back to back): 500 epochs 180 / 110 us, 10,000 204 / 132, 20,011 210 / 138, 40,000 206 / 136;
+// 56,000 153 in whole tiles, 161 in half ones.  (The queue of a packed batch takes whole tiles: the
+// same split there gave 6 % to twelve requests and cost 1 % of a full batch.)
+constexpr int kSplitHalfWaves = 5;
 constexpr int kMaxStage = 7000;  // staged samples: nsc + kTE - 1
 
 // One curve as a tile sees it: sample s at lc[s*stride], epoch e's outputs at [e*ostride].
@@ -106,8 +114,9 @@ __device__ __forceinline__ float df_sumsq(float bh, float bl, float ah, float al
   return __fadd_rn(s3, ((e3 + e2) + (ql - tl)) + ul);
 }
 
-// kTE consecutive epochs [e0, e0 + kTE) of one curve, by the whole block.
-__device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0) {
+// Halves [h0, h0 + n_halves) of the kTE consecutive epochs from e0 of one curve, by the whole block.
+// The whole tile's samples are staged either way, so that an epoch's result is the same to the bit.
+__device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const int h0, const int n_halves) {
   extern __shared__ __align__(16) float st[];
   __shared__ float red_sn[kWarps][kTE], red_l[kWarps][kTE], red_h[kWarps][kTE];
   __shared__ int red_w[kWarps][kTE];
@@ -250,10 +259,10 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0) {
     red_l[warp][32 * h + lane] = 0.0f;
     red_h[warp][32 * h + lane] = 0.0f;
   }
-  for (int u = warp; u < kHalves * a.nw; u += kWarps) {
+  for (int u = warp; u < n_halves * a.nw; u += kWarps) {
     const int half = u / a.nw;
     const int wi = (half & 1) ? (half + 1) * a.nw - 1 - u : u - half * a.nw;
-    const int e = e0 + 32 * half + lane;
+    const int e = e0 + 32 * (h0 + half) + lane;
     const bool eok = e < a.nt;
     const float ef = (float)e;
     const float dte = __fmul_rn(a.deltat, ef);
@@ -408,9 +417,9 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0) {
     }
   }
   __syncthreads();
-  if (warp < kHalves) {
+  if (warp < n_halves) {
     const int r = 32 * warp + lane;
-    const int e = e0 + r;
+    const int e = e0 + 32 * h0 + r;
     if (e < a.nt) {
       float best_sn = 0.0f, best_l = 0.0f, best_h = 0.0f;
       int best_w = INT_MAX;
@@ -434,18 +443,22 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0) {
   }
 }
 
-// Plain launch over an [n, nq] image: block = (epoch tile, curve), curves fastest.
+// Plain launch over an [n, nq] image: block = (epoch tile, curve, part of the tile), parts and then
+// curves fastest.
+template <int kParts>
 __global__ void __launch_bounds__(kTlsThreads, GTRAP_TLS_MINB) gtls_kernel(const TlsArgs img, const int nq) {
   __shared__ TlsArgs v;
-  const int tile = blockIdx.x / nq;
-  const int q = blockIdx.x - tile * nq;
+  const int item = blockIdx.x / kParts, part = blockIdx.x - item * kParts;
+  const int tile = item / nq;
+  const int q = item - tile * nq;
+  if (tile * kTE + part * (kTE / kParts) >= img.nt) return;   // no epoch left in the part
   if (threadIdx.x == 0) {
     v = img;
     v.lc += q; v.tu += q;
     v.sn += q; v.w += q; v.t0 += q; v.l += q; v.h += q;
   }
   __syncthreads();
-  gtls_tile(v, tile * kTE);
+  gtls_tile(v, tile * kTE, part, kHalves / kParts);
 }
 
 // Persistent launch over a device work queue of (curve, epoch tile) items of a packed batch.
@@ -488,7 +501,7 @@ __global__ void __launch_bounds__(kTlsThreads, GTRAP_TLS_MINB) gtls_queue_kernel
       v.mode = qa.mode; v.w_fma = qa.w_fma; v.t_fma = qa.t_fma; v.fix_a = qa.fix_a;
     }
     __syncthreads();
-    gtls_tile(v, e0);
+    gtls_tile(v, e0, 0, kHalves);
   }
 }
 
@@ -518,8 +531,10 @@ int gtrap_gtls(float *tlssn, float *tlsw, float *tlst0, float *tlsl, float *tlsh
   if (!(deltat > 0.0f)) return fail(GTRAP_ERR_INVALID_ARG, "gtls: deltat must be positive");
   const long long tiles = ((long long)nt + kTE - 1) / kTE;
   if (tiles * nq >= (1LL << 31)) return fail(GTRAP_ERR_INVALID_ARG, "gtls: grid too large");
+  const bool split = 2 * kHalves * tiles * nq <= (long long)kSplitHalfWaves * GTRAP_TLS_MINB * gtrap::sm_count();
+  const void *kernel = split ? (const void *)gtls_kernel<kHalves> : (const void *)gtls_kernel<1>;
   const size_t smem = tls_smem(nsc, nw);
-  GTRAP_TRY(gtrap::ensure_smem((const void *)gtls_kernel, smem, "gtls"));
+  GTRAP_TRY(gtrap::ensure_smem(kernel, smem, "gtls"));
   TlsArgs ta;
   ta.sn = tlssn; ta.w = tlsw; ta.t0 = tlst0; ta.l = tlsl; ta.h = tlshmax;
   ta.lc = lc; ta.tu = tu;
@@ -529,7 +544,10 @@ int gtrap_gtls(float *tlssn, float *tlsw, float *tlst0, float *tlsl, float *tlsh
   ta.w_fma = (flags & GTRAP_TLS_W_NOFMA) ? 0 : 1;
   ta.t_fma = (flags & GTRAP_TLS_T_NOFMA) ? 0 : 1;
   ta.fix_a = (flags & GTRAP_TLS_FIX_A) ? 1 : 0;
-  gtls_kernel<<<(unsigned)(tiles * nq), kTlsThreads, smem, stream>>>(ta, nq);
+  if (split)
+    gtls_kernel<kHalves><<<(unsigned)(tiles * nq * kHalves), kTlsThreads, smem, stream>>>(ta, nq);
+  else
+    gtls_kernel<1><<<(unsigned)(tiles * nq), kTlsThreads, smem, stream>>>(ta, nq);
   return gtrap::check_launch("gtls_kernel");
 }
 

@@ -112,3 +112,24 @@ def test_gtls_signal_found(cuda):
         ph = (t[e] - ep + 0.5 * per) % per - 0.5 * per if np.isfinite(t[e]) else 1e9
         hits += abs(ph) < inj[q, 3]
     assert hits >= 0.8 * strong.sum()
+
+
+@pytest.mark.parametrize("nt", [1, 31, 32, 33, 64, 65, 100, 1000])
+@pytest.mark.parametrize("nw", [1, 3, 8])
+def test_gtls_half_tiles(cuda, nt, nw):
+    """A small launch takes a tile as two blocks of half its epochs: the same bits as the curve gets in
+    an image that fills the GPU with whole tiles, with the last tile cut in either half."""
+    rng = np.random.default_rng(nt + nw)
+    n, nq = 1100, 120
+    t = ((np.arange(n) + 0.5) * synth.TESS_CADENCE).astype(np.float32)
+    t[200:260] = -1000.0
+    x = rng.normal(0, 1e-3, n).astype(np.float32)
+    g = synth.tls_grid(nw=nw, nl=5)
+
+    def run(k, m):
+        lc = torch.from_numpy(np.repeat(x[:, None], k, 1)).to(cuda)
+        tu = torch.from_numpy(np.repeat(t[:, None], k, 1)).to(cuda)
+        return api.gtls(lc, tu, m, g["nw"], g["nl"], g["nsc"], g["wmax"], g["dw"], g["deltat"])
+    for one, many in zip(run(1, nt), run(nq if nt == 1000 else 64 * nq, nt)):
+        assert torch.equal(one[:, 0].view(torch.int32), many[:, 0].view(torch.int32))
+        assert torch.equal(one[:, 0].view(torch.int32), many[:, -1].view(torch.int32))
