@@ -29,7 +29,7 @@ namespace {
 using gtrap::fail;
 using gtrap::frac64;
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 384;
 constexpr int kMaxFine = 4096;        // fine bins of one neighbourhood, (p2 - p1 + 1 + 2M) * S
 constexpr double kXqMax = 1099511627776.0;  // |quantised flux| < 2^40
 constexpr int kMaxGroup = 33;               // trials per block at most
@@ -245,10 +245,12 @@ __device__ __forceinline__ float ll_mag(long long v) {
 // takes a trial at a time.  G is what the neighbourhood leaves room for (wider ones take more
 // shared memory), less where there are too few curves to fill the SMs.  Bound by the phase and
 // histogram work of the samples; the FP64 powers are kept to the windows that FP32 bounds leave
-// (64 curves of 18,000 samples, 65 trials each: 893 -> 303 us, of which the fold takes 200; three
-// trials a block, every block finding peak and scale again, every window twice and 64-bit
-// compare-and-swap atomics before).
-__global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a) {
+// (64 curves of 18,000 samples, 65 trials each: 893 us with three trials a block, every block
+// finding peak and scale again, every window twice and 64-bit compare-and-swap atomics; 303 us with
+// those gone; 230 us with a shift for the fine bin where S is a power of two, windows screened
+// by a product and no quotient, and 12 warps a block for 8: 256 threads take 243 us, 512 (fewer
+// registers each) 275 us).
+__global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ long long shl[kThreads / 32];
   const uint32_t c = blockIdx.x;
@@ -297,33 +299,33 @@ __global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a)
   __syncthreads();
   const double unscale = ldexp(1.0, -sx);
   const uint32_t nbS = a.nb * S;
+  const bool pow2 = (S & (S - 1)) == 0;
+  const int fine_shift = 1 + __clz(nbS);   // 32 - log2(nb S)
   const Scale sc(sx);
   long long stot = 0;
-  constexpr int kU = 4;
-  for (uint32_t i0 = 0; i0 < cv.n; i0 += kThreads * kU) {   // kU samples' loads ahead of their uses
-    float tv[kU], xv[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const uint32_t i = i0 + u * kThreads + tid;
-      const size_t idx = cv.off + (size_t)i * cv.stride;
-      tv[u] = i < cv.n ? __ldg(a.t + idx) : -1.0f;
-      xv[u] = i < cv.n ? __ldg(a.x + idx) : 0.0f;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      if (!off_ok || !valid(tv[u], xv[u])) continue;
-      const long long xq = quantise(xv[u], cv.offset, sc);
-      stot += xq;
-      const unsigned xlo = (unsigned)xq & 0xfffffu, xhi = (unsigned)(xq >> 20);
-      const unsigned long long bp = frac64(tv[u], dfK);
-      unsigned long long ph = frac64(tv[u], cv.fmin) + (unsigned long long)J0 * bp - shift0 - lo;
-      const unsigned long long step = bp - Rp;
+  float tn, xn;
+  auto load = [&](uint32_t i) {   // a sample ahead of its use
+    const size_t idx = cv.off + (size_t)i * cv.stride;
+    tn = i < cv.n ? __ldg(a.t + idx) : -1.0f;
+    xn = i < cv.n ? __ldg(a.x + idx) : 0.0f;
+  };
+  load(tid);
+  for (uint32_t i = tid; i < cv.n; i += kThreads) {
+    const float tv = tn, xv = xn;
+    load(i + kThreads);
+    if (!off_ok || !valid(tv, xv)) continue;
+    const long long xq = quantise(xv, cv.offset, sc);
+    stot += xq;
+    const unsigned xlo = (unsigned)xq & 0xfffffu, xhi = (unsigned)(xq >> 20);
+    const unsigned long long bp = frac64(tv, dfK);
+    unsigned long long ph = frac64(tv, cv.fmin) + (unsigned long long)J0 * bp - shift0 - lo;
+    const unsigned long long step = bp - Rp;
+    // fine bin from the neighbourhood start: floor(ph nb S / 2^64), nb S < 2^20 (S a power of two: a shift)
+    auto trials = [&](auto bin) {
       uint32_t row = 0;
 #pragma unroll 4
       for (uint32_t g = 0; g < nk; ++g, ph += step, row += E) {
-        // fine bin from the neighbourhood start: floor(ph nb S / 2^64), nb S < 2^20
-        const uint32_t fb = (uint32_t)(((ph >> 32) * nbS + (((ph & 0xffffffffull) * nbS) >> 32)) >> 32);
+        const uint32_t fb = bin(ph);
         if (fb < LS) {
           unsigned *h = reinterpret_cast<unsigned *>(hs + row + fb);
           atomicAdd(h, xlo);
@@ -331,7 +333,13 @@ __global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a)
           atomicAdd(hc + row + fb, 1);
         }
       }
-    }
+    };
+    if (pow2)
+      trials([&](unsigned long long p) { return (uint32_t)(p >> 32) >> fine_shift; });
+    else
+      trials([&](unsigned long long p) {
+        return (uint32_t)(((p >> 32) * nbS + (((p & 0xffffffffull) * nbS) >> 32)) >> 32);
+      });
   }
   stot = block_sum<long long>(stot, shl);
   __syncthreads();
@@ -433,26 +441,39 @@ __global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a)
     // (a float prefix near the underflow range would break the bounds: no screening there)
     float thr = 0.0f;
     if (sx < 100) {
-      float top = 0.0f, lower = 0.0f;
+      // a lower bound of the largest power: first from the windows around the grid's, then raised by every
+      // window whose upper bound reaches it; the rows with such a window are the only ones compared
+      // exactly.  One product compared a window instead of a quotient: this stage of 64 curves x 65
+      // trials, windows of up to 205 bins, took 150 and takes 90 us.
+      auto lower = [&](float2 A, float2 B) -> float {   // 0 where the window does not count
+        const float kk = B.y - A.y, den = kk * (Nf - kk);
+        const float sv = fabsf(B.x - A.x), low = fmaxf(sv - (e0 + sv * (1.0f / 4194304.0f)), 0.0f);
+        return kk > kkmi_f && den > 0.0f ? __fdividef(low * low, den) * (1.0f - 1.0f / 1048576.0f) : 0.0f;
+      };
+      const int g0 = (int)M, g1 = iL - (int)M;   // the grid's window
+      for (int q = lane; q < 9 * 9; q += 32) {
+        const int ws = g0 + q / 9 - 4, we = g1 + q % 9 - 4;
+        if (ws >= 0 && we <= iL && we - ws > kmi && we - ws <= kma) thr = fmaxf(thr, lower(P[ws], P[we]));
+      }
+      thr = warp_max(thr);
       for (int s = 0; s < iL; ++s) {
         const float2 A = P[s];
         const int wmax = min(kma, iL - s);
-        float rowmax = 0.0f;
+        bool hit = false;
+#pragma unroll 2
         for (int w = kmi + 1 + lane; w <= wmax; w += 32) {
           const float2 B = P[s + w];
-          const float phi = upper(A, B);
-          rowmax = fmaxf(rowmax, phi);
-          if (phi > top) {   // the lane's best bound so far: the lower bound of its window
-            top = phi;
-            const float kk = B.y - A.y, den = kk * (Nf - kk);
-            const float sv = fabsf(B.x - A.x), low = fmaxf(sv - (e0 + sv * (1.0f / 4194304.0f)), 0.0f);
-            lower = fmaxf(lower, __fdividef(low * low, den) * (1.0f - 1.0f / 1048576.0f));
+          const float kk = B.y - A.y, den = kk * (Nf - kk);
+          const float sv = fabsf(B.x - A.x), hi = sv + (e0 + sv * (1.0f / 4194304.0f));
+          if (kk > kkmi_f && den > 0.0f && hi * hi * (1.0f + 1.0f / 524288.0f) >= thr * den) {
+            hit = true;
+            thr = fmaxf(thr, lower(A, B));
           }
         }
-        rowmax = warp_max(rowmax);
-        if (lane == 0) R[s] = rowmax;
+        const bool any = __any_sync(0xffffffffu, hit);
+        if (any) thr = warp_max(thr);
+        if (lane == 0) R[s] = any ? 1.0f : 0.0f;
       }
-      thr = warp_max(lower);
     }
     __syncwarp();
     double bp = -1.0;
@@ -466,7 +487,7 @@ __global__ void __launch_bounds__(kThreads) refine_trial_kernel(const RefArgs a)
       }
     };
     for (int s0 = 0; s0 < iL; s0 += 32) {
-      const bool in = s0 + lane < iL && (sx >= 100 || R[s0 + lane] >= thr);
+      const bool in = s0 + lane < iL && (sx >= 100 || R[s0 + lane] > 0.0f);
       for (unsigned rows = __ballot_sync(0xffffffffu, in); rows; rows &= rows - 1) {
         const int s = s0 + __ffs(rows) - 1;
         const float2 A = P[s];
