@@ -215,3 +215,18 @@ def test_refine_crowded_fine_bins(cuda, n, period):
     many = np.tile(x[:, None], (1, 200)), np.tile(t[:, None], (1, 200))
     _, _, _, recs2 = _search_and_refine(*many, np.repeat(ntrue, 200), np.repeat(off, 200), g, cuda)
     assert all(r.tobytes() == recs[0].tobytes() for r in recs2)
+
+
+@pytest.mark.parametrize("fine", [1, 6, 16])
+def test_refine_fine_bins_per_bin(cuda, fine):
+    """Fine bins by a shift (a power of two a bin, none at all included) and by the product."""
+    resid, tu, ntrue, off, g, _ = _image_case(nq=2, n=5000, nf=512, seed=67)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    r, t, o, nt = d(resid), d(tu), d(off), d(ntrue.astype(np.int32))
+    sr, p1, p2 = api.geebls(r, t, o, nt, g["nf"], g["nb"], g["kma"], g["kmi"], g["kkmi"], g["fmin"], g["df"])
+    recs = api.refined_to_numpy(api.bls_refine(sr, p1, p2, r, t, o, nt, g["nb"], g["kma"], g["kmi"], g["kkmi"],
+                                              g["fmin"], g["df"], K=16, S=fine, M=4))
+    sr, p1, p2 = sr.cpu().numpy(), p1.cpu().numpy().view(np.uint32), p2.cpu().numpy().view(np.uint32)
+    for q in range(2):
+        _check(recs[q], OR.refine_curve(tu[:, q], resid[:, q], off[q], ntrue[q], sr[q], p1[q], p2[q], g["fmin"],
+                                        g["df"], g["nb"], g["kma"], g["kmi"], g["kkmi"], K=16, S=fine, M=4))
