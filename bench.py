@@ -379,15 +379,14 @@ def run_masked(args, rank, world, local_rank):
             "gpu_launches": 6 * args.steps,
             "clocks": clk}
     # the detrend of the same image (gfilter, r = 24): its HBM roofline (8 B a sample read
-    # and written) beside its rate; the sorted-window updates in shared memory bind it
+    # and written) beside its rate; the sorting networks' min / max bind it
     hbm, hbm_src = _hbm_peak_gbs()
     samples = lc.shape[0] * lc.shape[1]
     gbs = 8.0 * samples / (gf_ms / 1e3) / 1e9
     line["gfilter"] = {"ms": gf_ms, "samples_per_s": samples / (gf_ms / 1e3),
                        "hbm": {"achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                                "peak_source": hbm_src, "bytes_per_sample": 8},
-                       "bound": "compute: per-sample sorted-window updates in shared memory (binary search "
-                                "and shifts), not HBM"}
+                       "bound": "compute: min / max of the sorting networks in registers, not HBM"}
     if e2e:
         line["e2e"] = e2e
     if not args.no_cpu_baseline:
