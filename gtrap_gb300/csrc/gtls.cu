@@ -29,6 +29,13 @@
 // slot i - nSx while classifying slot i (include/gtls_simple.h:212-225 index cache[i]
 // with the loop counter); the depth H is formed with that sum, and so it is here unless
 // GTRAP_TLS_FIX_A asks for region A's own flux.  chi^2 uses region A's own flux in both.
+//
+// Bound by issue (over 90 % active): about 400 instructions a step of L and warp, half of them the
+// walks' seven samples or so.  What they load lies side by side (time and flux, the two words of
+// a prefix), a masked sample is known by its flux and not by two counts, and a shifted time is one
+// fused operation whichever rounding is asked for: 96 TESS-like curves of 18,000 epochs 3.46 -> 3.08 ms,
+// one of 20,011 140 -> 119 us (counts held as floats, S/N without its quotient and root where a
+// product shows it below the best, and invariant corners in registers gave nothing more).
 #include "common.cuh"
 
 #include <climits>
@@ -53,6 +60,8 @@ constexpr int kHalves = kTE / 32;
 // 56,000 153 in whole tiles, 161 in half ones.  (The queue of a packed batch takes whole tiles: the
 // same split there gave 6 % to twelve requests and cost 1 % of a full batch.)
 constexpr int kSplitHalfWaves = 5;
+// The staged flux of a masked sample: a NaN that no subtraction gives (those give the canonical one).
+constexpr int kMaskedX = 0x7fc0dead;
 constexpr int kMaxStage = 7000;  // staged samples: nsc + kTE - 1
 
 // One curve as a tile sees it: sample s at lc[s*stride], epoch e's outputs at [e*ostride].
@@ -129,12 +138,11 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
   const int base = max(first, 0);
   const int S = max(0, min(last, a.nt) - base);
 
-  float *tq = st;                        // [S] shifted-search time (filled over masks)
-  float *xv = tq + S;                    // [S] x - xref (0 when masked)
-  int *cnt = (int *)(xv + S);            // [S+1] valid-count prefix
-  float *pxh = (float *)(cnt + S + 1);   // [S+1] prefix of x (hi, lo)
-  float *pxl = pxh + S + 1;
-  float *pqh = pxl + S + 1;              // [S+1] prefix of x^2 (hi, lo)
+  float2 *px = reinterpret_cast<float2 *>(st);   // [S+1] prefix of x (hi, lo)
+  // [S] shifted-search time (filled over masks), x - xref (kMaskedX when masked)
+  float2 *tx = px + S + 1;
+  int *cnt = (int *)(tx + S);            // [S+1] valid-count prefix
+  float *pqh = (float *)(cnt + S + 1);   // [S+1] prefix of x^2 (hi, lo)
   float *pql = pqh + S + 1;
   float *dlw = pql + S + 1;              // [nw] ingress step L / mm of each width
 
@@ -159,8 +167,7 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     const float tqv = __fadd_rn(-1000.0f, __fadd_rn(tr, 1000.0f));
     const float x = __ldg(a.lc + idx);
     const bool ok = tqv >= 0.0f;
-    tq[s] = ok ? tqv : -INFINITY;
-    xv[s] = ok ? x : 0.0f;
+    tx[s] = make_float2(ok ? tqv : -INFINITY, ok ? x : 0.0f);
     cnt[s] = ok ? 1 : 0;
   }
   __syncthreads();
@@ -171,7 +178,7 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     // reference level: mean of the valid staged values (makes the moments well conditioned)
     float acc = 0.0f;
     int n = 0;
-    for (int s = lane; s < S; s += 32) { acc += xv[s]; n += cnt[s]; }
+    for (int s = lane; s < S; s += 32) { acc += tx[s].y; n += cnt[s]; }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -186,12 +193,12 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     float lastt = -INFINITY;
     for (int s = s0; s < s1; ++s) {
       if (cnt[s]) {
-        const float xc = __fsub_rn(xv[s], ref);
-        xv[s] = xc;
+        const float xc = __fsub_rn(tx[s].y, ref);
+        tx[s].y = xc;
         c += 1;
         sx = df_add(sx, DF{xc, 0.0f});
         sq = df_add(sq, df_from_prod(xc));
-        lastt = tq[s];
+        lastt = tx[s].x;
       }
     }
     // exclusive scan of the lane totals (count, sx, sq) and of the last valid time
@@ -224,23 +231,24 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     float ft = pt;
     for (int s = s0; s < s1; ++s) {
       cnt[s] = rc;  // cnt becomes the exclusive prefix
-      pxh[s] = rx.hi; pxl[s] = rx.lo; pqh[s] = rq.hi; pql[s] = rq.lo;
-      if (tq[s] != -INFINITY) {
-        const float xc = xv[s];
+      px[s] = make_float2(rx.hi, rx.lo); pqh[s] = rq.hi; pql[s] = rq.lo;
+      if (tx[s].x != -INFINITY) {
+        const float xc = tx[s].y;
         rc += 1;
         rx = df_add(rx, DF{xc, 0.0f});
         rq = df_add(rq, df_from_prod(xc));
-        ft = tq[s];
+        ft = tx[s].x;
       } else {
-        tq[s] = ft;  // masked: previous valid time keeps the search predicate monotone
+        // masked: previous valid time keeps the search predicate monotone
+        tx[s] = make_float2(ft, __int_as_float(kMaskedX));
       }
     }
     // the lane owning element S-1 (the only one with s1 == S and a non-empty chunk)
     // writes the total at index S
     if (s1 == S && s0 < s1) {
-      cnt[S] = rc; pxh[S] = rx.hi; pxl[S] = rx.lo; pqh[S] = rq.hi; pql[S] = rq.lo;
+      cnt[S] = rc; px[S] = make_float2(rx.hi, rx.lo); pqh[S] = rq.hi; pql[S] = rq.lo;
     }
-    if (S == 0 && lane == 0) { cnt[0] = 0; pxh[0] = pxl[0] = pqh[0] = pql[0] = 0.0f; }
+    if (S == 0 && lane == 0) { cnt[0] = 0; px[0] = make_float2(0.0f, 0.0f); pqh[0] = pql[0] = 0.0f; }
   }
   __syncthreads();
 
@@ -265,11 +273,9 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     const int e = e0 + 32 * (h0 + half) + lane;
     const bool eok = e < a.nt;
     const float ef = (float)e;
-    const float dte = __fmul_rn(a.deltat, ef);
-    auto tt = [&](int s) -> float {
-      const float v = tq[s];
-      return t_fma ? __fmaf_rn(-a.deltat, ef, v) : __fsub_rn(v, dte);
-    };
+    // v - deltat e by one fused operation, or with the product rounded first (times 1, so exactly)
+    const float sh_a = t_fma ? -a.deltat : -1.0f, sh_b = t_fma ? ef : __fmul_rn(a.deltat, ef);
+    auto tt = [&](int s) -> float { return __fmaf_rn(sh_a, sh_b, tx[s].x); };
     // scoop of epoch e in staged indices; c0 is scoop slot 0 (negative before the series)
     const int c0 = e - nsch - base;
     const int lo = max(e - nsch, 0) - base;
@@ -310,6 +316,10 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     };
     auto ub = [&](float tau) -> int { return search(tau, [&](int s) { return tt(s) > tau; }); };
     auto lb = [&](float tau) -> int { return search(tau, [&](int s) { return tt(s) >= tau; }); };
+    auto px_diff = [&](int b, int a_) -> float {
+      const float2 pb = px[b], pa = px[a_];
+      return df_diff(pb.x, pb.y, pa.x, pa.y);
+    };
     float best_sn = 0.0f, best_l = 0.0f, best_h = 0.0f;
     int best_w = INT_MAX;
     if (eok && lo < hi) do {
@@ -323,8 +333,8 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
     const float filfac = __fdiv_rn((float)N, __fdiv_rn(W, crit_w));
     if (!(filfac > 0.75f)) continue;
     const int Nw = cnt[ubE] - cnt[lbS];
-    const float m = Nw > 0 ? __fdiv_rn(df_diff(pxh[ubE], pxl[ubE], pxh[lbS], pxl[lbS]), (float)Nw) : 0.0f;
-    const float SxAE = df_diff(pxh[ubE], pxl[ubE], pxh[ubS], pxl[ubS]);
+    const float m = Nw > 0 ? __fdiv_rn(px_diff(ubE, lbS), (float)Nw) : 0.0f;
+    const float SxAE = px_diff(ubE, ubS);
     const float SSf = df_sumsq(pqh[ubE], pql[ubE], pqh[ubS], pql[ubS], m, SxAE, N);
     const float dl = dlw[wi];
     const float Wq = 0.25f * W;  // exact
@@ -342,35 +352,39 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
       const float tCD = -tBC, tDE = -tAB;
       while (bL > lo && tt(bL - 1) > tAB) {
         --bL;
-        if (cnt[bL + 1] != cnt[bL]) {
-          const float x = xv[bL], u = __fadd_rn(tt(bL), Wq);
+        const float x = tx[bL].y;
+        if (__float_as_int(x) != kMaskedX) {
+          const float u = __fadd_rn(tt(bL), Wq);
           ++nB; xB += x; uB += u; xuB = fmaf(x, u, xuB); uuB = fmaf(u, u, uuB);
         }
       }
       while (bR < hi && !(tt(bR) > tBC)) {
-        if (cnt[bR + 1] != cnt[bR]) {
-          const float x = xv[bR], u = __fadd_rn(tt(bR), Wq);
+        const float x = tx[bR].y;
+        if (__float_as_int(x) != kMaskedX) {
+          const float u = __fadd_rn(tt(bR), Wq);
           ++nB; xB += x; uB += u; xuB = fmaf(x, u, xuB); uuB = fmaf(u, u, uuB);
         }
         ++bR;
       }
       while (dL > lo && tt(dL - 1) > tCD) {
         --dL;
-        if (cnt[dL + 1] != cnt[dL]) {
-          const float x = xv[dL], v = __fsub_rn(tt(dL), Wq);
+        const float x = tx[dL].y;
+        if (__float_as_int(x) != kMaskedX) {
+          const float v = __fsub_rn(tt(dL), Wq);
           ++nD; xD += x; vD += v; xvD = fmaf(x, v, xvD); vvD = fmaf(v, v, vvD);
         }
       }
       while (dR < hi && !(tt(dR) > tDE)) {
-        if (cnt[dR + 1] != cnt[dR]) {
-          const float x = xv[dR], v = __fsub_rn(tt(dR), Wq);
+        const float x = tx[dR].y;
+        if (__float_as_int(x) != kMaskedX) {
+          const float v = __fsub_rn(tt(dR), Wq);
           ++nD; xD += x; vD += v; xvD = fmaf(x, v, xvD); vvD = fmaf(v, v, vvD);
         }
         ++dR;
       }
       if (!(L != 0.0f)) continue;  // L = 0: H = 0/0 in the reference, never accepted
       const int nC = cnt[dL] - cnt[bR];
-      const float SxC = df_diff(pxh[dL], pxl[dL], pxh[bR], pxl[bR]);
+      const float SxC = px_diff(dL, bR);
       const int nACE = N - nB - nD;
       const int nAE = nACE - nC;
       const float xAEC = (SxAE - xB - xD) - m * (float)nACE;
@@ -381,14 +395,14 @@ __device__ __forceinline__ void gtls_tile(const TlsArgs &a, const int e0, const 
         const int nA = cnt[bL] - cnt[ubS];
         const int nAx = bL - ubS;
         const int jlo = max(c0, 0), jhi = max(c0 + nAx, jlo);
-        float QA = df_diff(pxh[jhi], pxl[jhi], pxh[jlo], pxl[jlo]) + xr * (float)(cnt[jhi] - cnt[jlo]);
+        float QA = px_diff(jhi, jlo) + xr * (float)(cnt[jhi] - cnt[jlo]);
         if (nAx > nA) {  // masked slots inside A drop their partner's flux
           for (int i = 0; i < nAx; ++i) {
             const int j = c0 + i;
-            if (cnt[ubS + i + 1] == cnt[ubS + i] && j >= 0 && cnt[j + 1] != cnt[j]) QA -= xv[j] + xr;
+            if (cnt[ubS + i + 1] == cnt[ubS + i] && j >= 0 && cnt[j + 1] != cnt[j]) QA -= tx[j].y + xr;
           }
         }
-        const float xA = df_diff(pxh[bL], pxl[bL], pxh[ubS], pxl[ubS]) - m * (float)nA;
+        const float xA = px_diff(bL, ubS) - m * (float)nA;
         xAEC_h = (xAEC - xA) + (QA - (m + xr) * (float)nA);
       }
       const float XU = xuB - m * uB;
