@@ -160,7 +160,22 @@ __device__ __forceinline__ long long entry_g(long long y, uint32_t lo) {
 // pbytes; histogram f (nb flux words, then nb counts) at pbytes - 8 nb + 8 nb f.  Histogram 0 lies inside the moment arrays and is read into
 // registers before they are written; later histograms lie past them.  A frequency whose bins
 // need 64-bit flux sums refolds them into the first 8 nb bytes, below histogram 0.
-template <int F, int RM, class Item>
+// Packed entries (PACK): GS modulo 2^48 | low half of G << 48, K | high half of G << 48: sixteen bytes and
+// four wavefronts a corner where 2 N E < 2^32 (G fits) and N dmax < 2^27 (every template's sum S w
+// fits 48 bits signed).  The templates are bound by the loads of their three corners (15 wavefronts a
+// warp without: 16 curves of 18,000 samples, 8192 periods, 2048 bins 7966 -> 7441 us; 4096 bins
+// 429 -> 399, 512 bins 116 -> 112).  Images only: a queue's curves differ in N.
+__device__ __forceinline__ longlong2 pack_entry16(long long gs, long long k, long long g) {
+  const unsigned long long gu = (unsigned long long)g;
+  return make_longlong2((long long)(((unsigned long long)gs & kM48) | gu << 48),
+                        (long long)((unsigned long long)k | (gu >> 16 & 0xffffu) << 48));
+}
+__device__ __forceinline__ uint32_t entry_g16(longlong2 e) {
+  return __byte_perm((uint32_t)((unsigned long long)e.x >> 32), (uint32_t)((unsigned long long)e.y >> 32), 0x7632);
+}
+__device__ __forceinline__ long long signed48(unsigned long long v) { return (long long)(v << 16) >> 16; }
+
+template <int F, int RM, bool PACK, class Item>
 __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ long long wsum[4][kTfWarps];
@@ -316,7 +331,7 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
       const long long x = b0;
       long long pc = c, m1 = x * c - ((cu - c) >> 1), kk = 4 * x * x * c - 4 * x * cu + cu2;
       long long ps = s, ms1 = x * s - ((su - s) >> 1);
-      if (tid == 0) { GSK[0] = make_longlong2(0, 0); Glo[0] = 0u; }
+      if (tid == 0) { GSK[0] = make_longlong2(0, 0); if (!PACK) Glo[0] = 0u; }
       longlong2 ent[RM];
       uint32_t glo[RM];
 #pragma unroll
@@ -324,7 +339,7 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
         kk += (long long)vc[r] + 8 * m1;
         pc += vc[r]; m1 += pc;
         ps += vs[r]; ms1 += ps;
-        ent[r] = pack_entry(2 * ms1 - ps, kk, 2 * m1 - pc);
+        ent[r] = PACK ? pack_entry16(2 * ms1 - ps, kk, 2 * m1 - pc) : pack_entry(2 * ms1 - ps, kk, 2 * m1 - pc);
         glo[r] = (uint32_t)(2 * m1 - pc);
       }
       if (RM == 2 || RM == 4) {
@@ -341,12 +356,12 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
             if (c2 == t) w = glo[t];
           }
           GSK[b0 + c + 1] = v;
-          Glo[b0 + c2 + 1] = w;
+          if (!PACK) Glo[b0 + c2 + 1] = w;
         }
       } else {
 #pragma unroll
         for (int r = 0; r < RM; ++r)
-          if (RM > 1 || b0 + r < nb) { GSK[b0 + r + 1] = ent[r]; Glo[b0 + r + 1] = glo[r]; }
+          if (RM > 1 || b0 + r < nb) { GSK[b0 + r + 1] = ent[r]; if (!PACK) Glo[b0 + r + 1] = glo[r]; }
       }
     }
     const long long Tc = (long long)wbasec[kTfWarps], Ts = wbase[0][kTfWarps];
@@ -354,13 +369,14 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
     // extension past nb: entry nb + e from entry e and the full-cycle sums
     {
       const longlong2 sn = GSK[nb];
-      const long long gn = entry_g(sn.y, Glo[nb]), kn = entry_k(sn.y);
+      const long long gn = PACK ? (long long)entry_g16(sn) : entry_g(sn.y, Glo[nb]), kn = entry_k(sn.y);
       for (int e = tid + 1; e <= (int)a.dmax; e += kTfThreads) {
         const long long e2 = 2LL * e;
         const longlong2 se = GSK[e];
-        const long long g = gn + e2 * Tc + entry_g(se.y, Glo[e]);
-        GSK[nb + e] = pack_entry(sn.x + e2 * Ts + se.x, kn + 2 * e2 * gn + e2 * e2 * Tc + entry_k(se.y), g);
-        Glo[nb + e] = (uint32_t)g;
+        const long long g = gn + e2 * Tc + (PACK ? (long long)entry_g16(se) : entry_g(se.y, Glo[e]));
+        const long long gs = sn.x + e2 * Ts + se.x, k = kn + 2 * e2 * gn + e2 * e2 * Tc + entry_k(se.y);
+        GSK[nb + e] = PACK ? pack_entry16(gs, k, g) : pack_entry(gs, k, g);   // (modulo 2^48 where packed)
+        if (!PACK) Glo[nb + e] = (uint32_t)g;
       }
     }
     __syncthreads();
@@ -377,7 +393,7 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
     for (int r = 0; r < RM; ++r) {
       const int i = min(tid + r * kTfThreads, nb - 1);
       si[r] = GSK[i];
-      gi[r] = Glo[i];
+      gi[r] = PACK ? entry_g16(si[r]) : Glo[i];
     }
     for (int d = 0; d < nd; ++d) {
       const int DL = sDL[f][d];
@@ -390,13 +406,15 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
         if (RM == 1 && i >= nb) break;
         const int e1 = i + L, e2 = i + D - L, e3 = i + D;
         const longlong2 c1 = GSK[e1], c2 = GSK[e2], c3 = GSK[e3];
-        const uint32_t l1 = Glo[e1], l2 = Glo[e2];
+        const uint32_t l1 = PACK ? entry_g16(c1) : Glo[e1], l2 = PACK ? entry_g16(c2) : Glo[e2];
         // sum C w < dmax N < 2^32: exact in 32-bit wrap-around arithmetic
-        const uint32_t A2 = gi[r] - l1 - l2 + Glo[e3];
-        const long long N2 = si[r].x - c1.x - c2.x + c3.x;
+        const uint32_t A2 = gi[r] - l1 - l2 + (PACK ? entry_g16(c3) : Glo[e3]);
+        const long long X = si[r].x - c1.x - c2.x + c3.x;
+        const long long N2 = PACK ? signed48((unsigned long long)X) : X;
         // sum C w^2 < N dmax^2 < 2^44: exact modulo 2^48, so the packed words combine directly
+        const long long g12 = PACK ? (long long)l1 + (long long)l2 : entry_g(c1.y, l1) + entry_g(c2.y, l2);
         const long long B4 = (long long)(((unsigned long long)(c3.y - c2.y + c1.y - si[r].y) -
-                                          (unsigned long long)(L4 * (entry_g(c1.y, l1) + entry_g(c2.y, l2)))) & kM48);
+                                          (unsigned long long)(L4 * g12)) & kM48);
         const float a2 = (float)A2;
         const float num = i64_to_f32(N2) - mean * a2;
         const float den = Nf * i64_to_f32(B4) - a2 * a2;
@@ -427,9 +445,11 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
         const int DL = sDL[f][d], D = DL & 0xffff, L = DL >> 16;
         const int e1 = i + L, e2 = i + D - L, e3 = i + D;
         const longlong2 c0 = GSK[i], c1 = GSK[e1], c2 = GSK[e2], c3 = GSK[e3];
-        const long long g1 = entry_g(c1.y, Glo[e1]), g2 = entry_g(c2.y, Glo[e2]);
-        const long long A2 = entry_g(c0.y, Glo[i]) - g1 - g2 + entry_g(c3.y, Glo[e3]);
-        const long long N2 = c0.x - c1.x - c2.x + c3.x;
+        auto g_of = [&](longlong2 c, int x) { return PACK ? (long long)entry_g16(c) : entry_g(c.y, Glo[x]); };
+        const long long g1 = g_of(c1, e1), g2 = g_of(c2, e2);
+        const long long A2 = g_of(c0, i) - g1 - g2 + g_of(c3, e3);
+        const long long X = c0.x - c1.x - c2.x + c3.x;
+        const long long N2 = PACK ? signed48((unsigned long long)X) : X;
         const long long B4 = entry_k(c3.y) - entry_k(c2.y) + entry_k(c1.y) - entry_k(c0.y) - 4LL * L * (g1 + g2);
         const double num = (double)N2 - (double)mean * (double)A2;
         const double den = (double)Nf * (double)B4 - (double)A2 * (double)A2;
@@ -443,10 +463,10 @@ __device__ __forceinline__ void tf_item(const TfShape &a, const Item &c) {
   }
 }
 
-template <int F, int RM>
+template <int F, int RM, bool PACK>
 __global__ void __launch_bounds__(kTfThreads, 2) tlsfold_kernel(const TfArgs a) {
   const uint32_t q = blockIdx.x / a.ngroups;
-  tf_item<F, RM>(a.sh, ImgItem{a, q, (blockIdx.x - q * a.ngroups) * F});
+  tf_item<F, RM, PACK>(a.sh, ImgItem{a, q, (blockIdx.x - q * a.ngroups) * F});
 }
 
 // Persistent blocks pop items from the device counter.  The barrier at the top of the loop
@@ -482,7 +502,7 @@ __global__ void __launch_bounds__(kTfThreads, 2) tlsfold_queue_kernel(const TfSh
     const int state = item.state;
     if (state == 2) break;
     if (state == 1) continue;
-    tf_item<F, RM>(sh, QueueItem{item, qa.tsr, qa.depth, qa.start, qa.dur});
+    tf_item<F, RM, false>(sh, QueueItem{item, qa.tsr, qa.depth, qa.start, qa.dur});
   }
 }
 
@@ -502,12 +522,17 @@ int tf_slot(int rm) { return rm == 1 ? 0 : rm == 2 ? 1 : rm == 4 ? 2 : 3; }
 int tf_rm(uint32_t nb) { return nb >= 4096 ? 8 : nb >= 2048 ? 4 : nb >= 1024 ? 2 : 1; }
 
 // nb = 4096 (8 bins a thread) leaves no room for a second histogram at two blocks an SM
-TfKernel tf_kernel(int F, int rm) {
+template <bool PACK>
+TfKernel tf_kernel_of(int F, int rm) {
   static const TfKernel table[kTfMaxF][4] = {
-      {tlsfold_kernel<1, 1>, tlsfold_kernel<1, 2>, tlsfold_kernel<1, 4>, tlsfold_kernel<1, 8>},
-      {tlsfold_kernel<2, 1>, tlsfold_kernel<2, 2>, tlsfold_kernel<2, 4>, nullptr},
-      {tlsfold_kernel<3, 1>, tlsfold_kernel<3, 2>, tlsfold_kernel<3, 4>, nullptr}};
+      {tlsfold_kernel<1, 1, PACK>, tlsfold_kernel<1, 2, PACK>, tlsfold_kernel<1, 4, PACK>, tlsfold_kernel<1, 8, PACK>},
+      {tlsfold_kernel<2, 1, PACK>, tlsfold_kernel<2, 2, PACK>, tlsfold_kernel<2, 4, PACK>, nullptr},
+      {tlsfold_kernel<3, 1, PACK>, tlsfold_kernel<3, 2, PACK>, tlsfold_kernel<3, 4, PACK>, nullptr}};
   return table[F - 1][tf_slot(rm)];
+}
+
+TfKernel tf_kernel(int F, int rm, bool pack = false) {
+  return pack ? tf_kernel_of<true>(F, rm) : tf_kernel_of<false>(F, rm);
 }
 
 TfQueueKernel tf_queue_kernel(int F, int rm) {
@@ -598,7 +623,9 @@ int gtrap_tls_fold(float *tsr, uint32_t *start, uint32_t *dur, float *depth, con
   const int F = pick_F(nb, dmax);
   a.ngroups = (nf + F - 1) / F;
   if ((uint64_t)nq * a.ngroups >= (1ull << 31)) return fail(GTRAP_ERR_INVALID_ARG, "tls_fold: nq*nf too large");
-  const TfKernel k = tf_kernel(F, tf_rm(nb));
+  // G < 2 N E and |sum S w| < N dmax 2^20 fit the packed entries' 32 and 48 bits (n bounds N)
+  const bool pack = 2ull * n * ((uint64_t)nb + dmax + 1) < (1ull << 32) && (uint64_t)n * dmax < (1ull << 27);
+  const TfKernel k = tf_kernel(F, tf_rm(nb), pack);
   const size_t smem = tf_smem(nb, dmax, F);
   GTRAP_TRY(ensure_smem((const void *)k, smem, "tls_fold"));
   k<<<(unsigned)(nq * a.ngroups), kTfThreads, smem, stream>>>(a);

@@ -75,3 +75,23 @@ def test_tls_fold_recovers_injected_period(cuda):
     j = int(torch.argmax(tsr[0]))
     assert abs(1.0 / (fmin + j * df) - per) < 0.01
     assert float(dep[0, j]) == pytest.approx(depth, rel=0.3)
+
+
+@pytest.mark.parametrize("n,nb,dmax,lfrac", [(32000, 4096, 4096, 0.5), (20000, 2048, 1024, 0.2), (3000, 512, 256, 0.3)])
+def test_tls_fold_packed_entries(cuda, n, nb, dmax, lfrac):
+    """Curves short enough for packed moment entries, and the same curves followed by masked samples that
+    make the image too long for them: the same bits, up to the largest sums of the packed form."""
+    rng = np.random.default_rng(n)
+    extra = (1 << 27) // dmax + 1 - n
+    t = ((np.arange(n) + 0.5) * synth.TESS_CADENCE).astype(np.float32)
+    x = np.stack([rng.normal(0, 1e-3, n), np.where(t % 2.0 < 1.0, 1.0, -1.0)], 1).astype(np.float32)
+    x[n // 4: n // 4 + 50, 0] -= 5e-3
+    tu = np.repeat(t[:, None], 2, 1)
+
+    def run(pad):
+        lc = np.concatenate([x, np.zeros((pad, 2), np.float32)])
+        tt = np.concatenate([tu, np.full((pad, 2), -1000.0, np.float32)])
+        d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+        return api.tls_fold(d(lc), d(tt), torch.zeros(2, device=cuda), 30, nb, 0.3, 0.05, W, lfrac=lfrac, dmax=dmax)
+    for a, b in zip(run(0), run(extra)):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
