@@ -1237,10 +1237,10 @@ def run_tlsfold(args, rank, world, local_rank):
     if rank != 0:
         return
     # roofline: the template phase reads the moment entries from shared memory; per template
-    # three corners of 16 + 4 bytes (GS, K with the high word of G, low word of G) = 60 B,
+    # three corners of 16 bytes (GS, K and G packed: this image's length allows it) = 48 B,
     # plus 20 B per start bin and frequency for the start corner
     tpl = float(tlsfold_valid_templates().sum()) * nq * TF_NB
-    lds_bytes = tpl * 60.0 + float(evals) * TF_NB * 20.0
+    lds_bytes = tpl * 48.0 + float(evals) * TF_NB * 16.0
     speak = smem_load_peak(dev)
     achieved = lds_bytes / (ms / 1e3)
     nv = float(np.count_nonzero(np.isfinite(lcn) & (tun >= 0)))
@@ -1260,7 +1260,7 @@ def run_tlsfold(args, rank, world, local_rank):
                          "frac": achieved / speak, "traffic": traffic,
                          "kernel": "tlsfold_kernel (fold + moment arrays + templates)",
                          "kernel_ms": ms, "templates_per_step": tpl,
-                         "algorithmic_bytes": "60 B of shared-memory loads per template + 20 B per "
+                         "algorithmic_bytes": "48 B of shared-memory loads per template + 16 B per "
                                               "start bin and frequency",
                          "peak_source": "live probe: conflict-free 64-bit shared-memory loads",
                          "fold": fold_leg},
