@@ -1238,7 +1238,7 @@ def run_tlsfold(args, rank, world, local_rank):
         return
     # roofline: the template phase reads the moment entries from shared memory; per template
     # three corners of 16 bytes (GS, K and G packed: this image's length allows it) = 48 B,
-    # plus 20 B per start bin and frequency for the start corner
+    # plus 16 B per start bin and frequency for the start corner
     tpl = float(tlsfold_valid_templates().sum()) * nq * TF_NB
     lds_bytes = tpl * 48.0 + float(evals) * TF_NB * 16.0
     speak = smem_load_peak(dev)
