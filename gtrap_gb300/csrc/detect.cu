@@ -15,6 +15,7 @@
 // reference's unstable argsort leaves their order open.  The survivors are written in
 // increasing index order.
 #include "common.cuh"
+#include "peakstate.cuh"
 
 #include <cooperative_groups.h>
 #include <math.h>
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(kDpThreads) detect_peaks_kernel(const DpArgs a
 
 constexpr int kDcRanks = 8;
 constexpr int kDcAhead = 8;          // words of states a warp compacts at once
-constexpr uint64_t kDcMinN = 64;     // the states' words must fit the byte a sample of the caller's
+constexpr uint64_t kDcMinN = 64;     // 7 bytes of alignment and n / 32 + 3 words fit the caller's byte a sample
 constexpr uint64_t kDcMaxN = 0x7fffffff;
 
 // Doubles are compared as integers (an FP64 instruction takes a warp 16 cycles or more here): keys
@@ -158,14 +159,24 @@ __device__ __forceinline__ long long dp_key(long long b) {
   return b < 0 ? b ^ 0x7fffffffffffffffll : b;
 }
 
+// A word of states is read by warps of every block while its own warp writes it: one access each, at L2.
+__device__ __forceinline__ uint64_t load_word(const uint64_t *p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_word(uint64_t *p, uint64_t v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 // Blocks 0 .. kDcRanks - 1 of one cluster.  Candidates are listed in index order (each block a
-// run of samples), their states kept as bits, and a round of the suppression compares the mask of a
-// candidate's higher neighbours with the states' bits around it, a warp taking 32 candidates: a
-// candidate is decided by candidates that rank above it alone.  Scratch: positions in the upper half
-// of the index output (peak k is written only when the positions up to the k-th candidate have been
-// read, which lie past it), masks in the lower half, states in `state`.  Bound by the latency of
-// the rounds and of the list steps.  One block, walking samples / the cluster, mpd 10: 20,011 samples
-// 777 / 33 us, 2^20 samples 40.6 / 0.75 ms; mpd 100: 3.9 / 0.27 ms, 135 / 5.1 ms.
+// run of samples), their states kept as bits (peakstate.cuh), and a round of the suppression compares
+// the mask of a candidate's higher neighbours with the states' bits around it, a warp taking 32
+// candidates: a candidate is decided by candidates that rank above it alone.  Scratch: positions in
+// the upper half of the index output (peak k is written only when the positions up to the k-th
+// candidate have been read, which lie past it), masks in the lower half, states in `state`.  Bound by
+// the latency of the rounds and of the list steps.  One block, walking samples / the cluster, mpd 10:
+// 20,011 samples 779 / 28 us, 2^20 samples 40.2 / 0.63 ms; mpd 100: 3.9 / 0.23 ms, 135 / 4.6 ms.
 __global__ void __cluster_dims__(kDcRanks, 1, 1) __launch_bounds__(kDpThreads, 1)
 detect_peaks_cluster_kernel(const DpArgs a) {
   namespace cg = cooperative_groups;
@@ -184,9 +195,8 @@ detect_peaks_cluster_kernel(const DpArgs a) {
   };
   unsigned *const list = reinterpret_cast<unsigned *>(a.out) + n;          // positions of the candidates
   unsigned *const higher = reinterpret_cast<unsigned *>(a.out);             // masks (bits 0-15 before, 16-31 behind)
-  const int64_t words = n / 32 + 3;
-  unsigned *const und = reinterpret_cast<unsigned *>(((uintptr_t)a.state + 3) & ~uintptr_t(3)) + 1;
-  unsigned *const kep = und + words;
+  // states of 32 candidates a word, a zero word on either side
+  uint64_t *const state = reinterpret_cast<uint64_t *>(((uintptr_t)a.state + 7) & ~uintptr_t(7)) + 1;
 
   cluster.sync();   // every block has started: its shared memory may be written
 
@@ -264,7 +274,7 @@ detect_peaks_cluster_kernel(const DpArgs a) {
   const int near = a.edge == 3 ? (int)min(w, (int64_t)17) : (int)(min(w, (int64_t)34) / 2);
   const bool masks = near <= 16;   // the entries within the window are among the 16 on either side
   const int64_t gwarp = (int64_t)rank * (kDpThreads / 32) + warp, nwarp = kDcRanks * (kDpThreads / 32);
-  if (gwarp == 0 && lane < 2) { const int64_t i = lane ? nword : -1; __stcg(und + i, 0u); __stcg(kep + i, 0u); }
+  if (gwarp == 0 && lane < 2) store_word(state + (lane ? nword : -1), 0u);
   for (int64_t i = gwarp; i < nword; i += nwarp) {
     const int64_t c = 32 * i + lane;
     unsigned m = w > 1 ? 1u : 0u;
@@ -285,7 +295,7 @@ detect_peaks_cluster_kernel(const DpArgs a) {
       __stcg(higher + c, m);
     }
     const unsigned u = __ballot_sync(0xffffffffu, c < M && m), k0 = __ballot_sync(0xffffffffu, c < M && !m);
-    if (lane == 0) { __stcg(und + i, u); __stcg(kep + i, k0); }
+    if (lane == 0) store_word(state + i, gtrap::peak_word(u, k0));
   }
   cluster.sync();
   // ---- rounds; each decides at least the highest undecided candidate
@@ -293,21 +303,15 @@ detect_peaks_cluster_kernel(const DpArgs a) {
     for (int64_t round = 0; round <= M; ++round) {
       int busy = 0;
       for (int64_t i = gwarp; i < nword; i += nwarp) {
-        const unsigned U = __ldcg(und + i);
+        const uint64_t own = load_word(state + i);   // (this warp alone writes it)
+        const unsigned U = gtrap::undecided_of(own);
         if (!U) continue;
         const bool mine = (U >> lane) & 1u;
         bool del = false, blocked = false;
         const int64_t c = 32 * i + lane;
-        const unsigned Kp = __ldcg(kep + i);
         if (masks) {
-          const unsigned m = mine ? __ldcg(higher + c) : 0u;
-          auto around = [&](const unsigned *b, unsigned mid) {   // bits of the 16 entries either side
-            const unsigned long long lo = ((unsigned long long)mid << 32) | __ldcg(b + i - 1);
-            const unsigned long long hi = ((unsigned long long)__ldcg(b + i + 1) << 32) | mid;
-            return ((unsigned)(lo >> (16 + lane)) & 0xffffu) | ((unsigned)(hi >> (lane + 1)) << 16);
-          };
-          blocked = m & around(und, U);
-          del = m & around(kep, Kp);
+          const uint64_t before = load_word(state + i - 1), behind = load_word(state + i + 1);
+          gtrap::peak_decide<16>(before, own, behind, mine ? __ldcg(higher + c) : 0u, lane, del, blocked);
         } else if (mine) {
           const unsigned e = __ldcg(list + c);
           const long long v = value(e);
@@ -315,7 +319,8 @@ detect_peaks_cluster_kernel(const DpArgs a) {
             const unsigned p = __ldcg(list + j);
             if ((p > e ? p - e : e - p) > w) return false;
             const unsigned bit = 1u << (j & 31);
-            const bool isu = __ldcg(und + (j >> 5)) & bit, isk = __ldcg(kep + (j >> 5)) & bit;
+            const uint64_t s = load_word(state + (j >> 5));
+            const bool isu = gtrap::undecided_of(s) & bit, isk = gtrap::kept_of(s) & bit;
             if ((isu || isk) && above(value(p), p, v, e)) {
               if (isk) del = true;
               else blocked = true;
@@ -327,11 +332,7 @@ detect_peaks_cluster_kernel(const DpArgs a) {
         }
         const unsigned kb = __ballot_sync(0xffffffffu, mine && !del && !blocked);
         const unsigned db = __ballot_sync(0xffffffffu, mine && del);
-        if (lane == 0 && (kb | db)) {   // kept before no longer undecided: nobody sees it as deleted in between
-          __stcg(kep + i, Kp | kb);
-          __threadfence();
-          __stcg(und + i, U & ~(kb | db));
-        }
+        if (lane == 0 && (kb | db)) store_word(state + i, gtrap::peak_word(U & ~(kb | db), gtrap::kept_of(own) | kb));
         busy |= (U & ~(kb | db)) != 0u;
       }
       busy = __syncthreads_or(busy);
@@ -349,7 +350,7 @@ detect_peaks_cluster_kernel(const DpArgs a) {
 #pragma unroll
     for (int u = 0; u < kDcAhead; ++u) {
       const int64_t i = w0 + (int64_t)warp * kDcAhead + u;
-      bits[u] = i < nword ? __ldcg(kep + i) : 0u;
+      bits[u] = i < nword ? gtrap::kept_of(load_word(state + i)) : 0u;
       pos[u] = (bits[u] >> lane) & 1u ? __ldcg(list + 32 * i + lane) : 0u;
       before[u] = mine;
       mine += __popc(bits[u]);
