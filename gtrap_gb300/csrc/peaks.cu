@@ -17,6 +17,7 @@
 //    median) / std; pssn = inf and diff = 0 when there are at most ntop peaks.
 // Medians are exact order statistics found by radix selection over the float bit patterns.
 #include "common.cuh"
+#include "peakstate.cuh"
 
 #include <math.h>
 
@@ -470,13 +471,11 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
     const uint32_t *__restrict__ len, size_t stride, uint32_t max_n, uint32_t mpd, uint32_t ntop, uint32_t k,
     gtrap_peak_stats *out, uint32_t *peak_idx, float *peak_val) {
   extern __shared__ __align__(16) float sv[];     // [max_n] the series
-  // candidates' states as bits (a word and a zero word on either side), their positions, and the
-  // kept peaks' positions (while the suppression runs: the masks of higher candidates)
-  const unsigned words = max_n / 64 + 3;
-  volatile unsigned *und = reinterpret_cast<unsigned *>(sv + max_n) + 1;
-  volatile unsigned *kep = und + words;
-  unsigned short *list = reinterpret_cast<unsigned short *>(sv + max_n) + 4 * words;   // [max_n / 2 + 1]
-  unsigned short *kept = list + max_n / 2 + 1;                                          // [max_n / 2 + 1]
+  // candidates' states (peakstate.cuh; a zero word on either side), their positions, and the kept
+  // peaks' positions (while the suppression runs: the masks of higher candidates)
+  volatile uint64_t *state = reinterpret_cast<uint64_t *>(sv + ((max_n + 1) & ~1u)) + 1;   // [-1 .. max_n / 64 + 1]
+  unsigned short *list = reinterpret_cast<unsigned short *>(sv + ((max_n + 1) & ~1u)) + 4 * (max_n / 64 + 3);
+  unsigned short *kept = list + max_n / 2 + 1;   // both [max_n / 2 + 1]
   __shared__ unsigned hist[kStBins];
   __shared__ StScratch sc;
   const int q = blockIdx.x, tid = threadIdx.x;
@@ -562,7 +561,7 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
   const int nword = (M + 31) >> 5;
   const bool masks = w > 0 && w <= 16;
   unsigned short *higher = kept;   // bit j: entry c - 8 + j (j < 8) or c - 7 + j
-  if (tid < 2) { const int i = tid ? nword : -1; und[i] = 0u; kep[i] = 0u; }
+  if (tid < 2) state[tid ? nword : -1] = 0u;
   for (int i = tid >> 5; i < nword; i += kStThreads / 32) {
     const int c = 32 * i + lane;
     unsigned m = w > 0 ? 1u : 0u;
@@ -578,27 +577,22 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
       higher[c] = (unsigned short)m;
     }
     const unsigned u = __ballot_sync(0xffffffffu, c < M && m), k0 = __ballot_sync(0xffffffffu, c < M && !m);
-    if (lane == 0) { und[i] = u; kep[i] = k0; }
+    if (lane == 0) state[i] = gtrap::peak_word(u, k0);
   }
   __syncthreads();
   if (w > 0) {
     for (int round = 0; round <= M; ++round) {
       int busy = 0;
       for (int i = tid >> 5; i < nword; i += kStThreads / 32) {
-        const unsigned U = und[i];
+        const uint64_t own = state[i];   // (this warp alone writes it)
+        const unsigned U = gtrap::undecided_of(own);
         if (!U) continue;
         const bool mine = (U >> lane) & 1u;
         bool del = false, blocked = false;
         const int c = 32 * i + lane;
         if (masks) {
-          const unsigned m = mine ? higher[c] : 0u;
-          auto around = [&](volatile unsigned *b, unsigned mid) {   // bits of the entries either side
-            const unsigned long long lo = ((unsigned long long)mid << 32) | b[i - 1];
-            const unsigned long long hi = ((unsigned long long)b[i + 1] << 32) | mid;
-            return ((unsigned)(lo >> (24 + lane)) & 0xffu) | (((unsigned)(hi >> (lane + 1)) & 0xffu) << 8);
-          };
-          blocked = m & around(und, U);
-          del = m & around(kep, kep[i]);
+          const uint64_t before = state[i - 1], behind = state[i + 1];
+          gtrap::peak_decide<8>(before, own, behind, mine ? higher[c] : 0u, lane, del, blocked);
         } else if (mine) {
           const int e = list[c];
           const float v = sv[e];
@@ -606,8 +600,9 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
             const int p = list[j];
             if (abs(p - e) > w) return false;
             const unsigned bit = 1u << (j & 31);
-            if (und[j >> 5] & bit) blocked |= prio_gt(sv[p], p, v, e);
-            else if (kep[j >> 5] & bit) del = true;
+            const uint64_t s = state[j >> 5];
+            if (gtrap::undecided_of(s) & bit) blocked |= prio_gt(sv[p], p, v, e);
+            else if (gtrap::kept_of(s) & bit) del = true;
             return true;
           };
           for (int j = c - 1; j >= 0 && !del && look(j); --j) {}
@@ -615,11 +610,7 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
         }
         const unsigned kb = __ballot_sync(0xffffffffu, mine && !del && !blocked);
         const unsigned db = __ballot_sync(0xffffffffu, mine && del);
-        if (lane == 0) {   // kept before no longer undecided: nobody sees it as deleted in between
-          kep[i] = kep[i] | kb;
-          __threadfence_block();
-          und[i] = U & ~(kb | db);
-        }
+        if (lane == 0) state[i] = gtrap::peak_word(U & ~(kb | db), gtrap::kept_of(own) | kb);
         busy |= (U & ~(kb | db)) != 0u;
       }
       if (!__syncthreads_or(busy)) break;
@@ -629,10 +620,10 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
   // the kept peaks as a list of their own, in index order
   {
     unsigned cnt = 0;
-    for (int i = tid; i < nword; i += kStThreads) cnt += __popc(kep[i]);   // (nword <= threads)
+    for (int i = tid; i < nword; i += kStThreads) cnt += __popc(gtrap::kept_of(state[i]));   // (nword <= threads)
     unsigned to = st_scan(cnt, sc);
     for (int i = tid; i < nword; i += kStThreads)
-      for (unsigned m = kep[i]; m; m &= m - 1) kept[to++] = list[32 * i + __ffs(m) - 1];
+      for (unsigned m = gtrap::kept_of(state[i]); m; m &= m - 1) kept[to++] = list[32 * i + __ffs(m) - 1];
   }
   __syncthreads();
   const unsigned K = sc.count;
@@ -689,7 +680,7 @@ __global__ void __launch_bounds__(kStThreads, 1) peakstat_staged_kernel(
 
 // Shared memory of a staged series: values, states and two lists of positions (candidates are
 // never adjacent, so at most half as many as samples).
-size_t staged_bytes(size_t max_n) { return 4 * max_n + 8 * (max_n / 64 + 3) + 4 * (max_n / 2 + 1); }
+size_t staged_bytes(size_t max_n) { return 4 * ((max_n + 1) & ~size_t(1)) + 8 * (max_n / 64 + 3) + 4 * (max_n / 2 + 1); }
 
 size_t staged_max() {
   const size_t room = (size_t)gtrap::max_smem_optin() - sizeof(StScratch) - kStBins * sizeof(unsigned) - 256;

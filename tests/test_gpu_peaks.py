@@ -117,3 +117,16 @@ def test_staged_and_long_series_agree(cuda, mpd, ntop, k):
         np.testing.assert_array_equal(a[key], b[key][:-1], err_msg=key)
     for key in ("std", "far", "pssn", "diff", "stdc"):
         np.testing.assert_allclose(a[key], b[key][:-1], rtol=1e-11, atol=1e-13, err_msg=key)
+
+
+@pytest.mark.parametrize("n", [3, 63, 64, 65, 66, 129, 4095, 8193, 35001])
+def test_states_at_word_edges(cuda, n):
+    """A lone series whose candidates just fill or just pass a word of states, odd and even lengths (the words
+    lie behind the series), windows of masks (up to 16 samples) and of lists, long chains of decisions."""
+    zigzag = np.zeros(n, np.float32)
+    zigzag[1::2] = 1.0 + np.arange(n // 2, dtype=np.float32) / 64.0
+    for x in (_series(60 + n, n), _series(61 + n, n), zigzag):
+        for mpd in (1, 2, 16, 17, 40):
+            st, idx, val = api.peakstat(torch.from_numpy(x).to(cuda), torch.zeros(1, dtype=torch.int64, device=cuda),
+                                        torch.full((1,), n, dtype=torch.int32, device=cuda), 1, n, mpd, 3, 16)
+            _check(api.stats_to_numpy(st)[0], idx.cpu().numpy()[0], val.cpu().numpy()[0], x, mpd, 3, 16)
