@@ -28,9 +28,12 @@ using gtrap::fail;
 constexpr int kPkThreads = 512;
 constexpr unsigned char kNone = 0, kUndecided = 1, kKept = 2, kDeleted = 3;
 
-__device__ __forceinline__ unsigned okey(float v) {  // order-preserving key of a float
+// Order-preserving key of a float.  NaN with the sign bit set ranks below all, without it as -0: one rule
+// for every order statistic here, whichever kernel a series runs on.  (Written out: with the sign bit put
+// into a float's bits by an or, the compiler's code gave that very key for such a NaN.)
+__device__ __forceinline__ unsigned okey(float v) {
   const unsigned b = __float_as_uint(v);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  return (b & 0x80000000u) ? ~b : b > 0x7f800000u ? 0x7fffffffu : (b | 0x80000000u);
 }
 __device__ __forceinline__ float okey_inv(unsigned k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
@@ -417,7 +420,6 @@ template <typename Val>
 __device__ __forceinline__ void st_select(Val val, unsigned n, unsigned k, unsigned step, unsigned *hist,
                                           StScratch &sc, float &a, float &b) {
   const int tid = threadIdx.x;
-  auto key_of = [](float v) { return isnan(v) ? 0u : okey(v); };   // NaN ranks lowest
   unsigned prefix = 0, mask = 0, left = k, same = 0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -428,7 +430,7 @@ __device__ __forceinline__ void st_select(Val val, unsigned n, unsigned k, unsig
     hist[tid + kStThreads] = 0;
     __syncthreads();
     for (unsigned e = tid; e < n; e += kStThreads) {
-      const unsigned u = key_of(val(e));
+      const unsigned u = okey(val(e));
       if ((u & mask) == prefix) atomicAdd(hist + ((u >> shift) & (bins - 1)), 1u);
     }
     __syncthreads();
@@ -450,7 +452,7 @@ __device__ __forceinline__ void st_select(Val val, unsigned n, unsigned k, unsig
     __syncthreads();
     unsigned m = 0xffffffffu;
     for (unsigned e = tid; e < n; e += kStThreads) {
-      const unsigned u = key_of(val(e));
+      const unsigned u = okey(val(e));
       if (u > prefix) m = min(m, u);
     }
     m = __reduce_min_sync(0xffffffffu, m);

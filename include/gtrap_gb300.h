@@ -443,7 +443,8 @@ typedef struct {
   uint32_t argmax;  /* first index of the maximum */
   uint32_t lent;    /* count of x > 0 */
   uint32_t npeaks;  /* peaks after the +-mpd suppression */
-  double median;    /* median(x), mean of the two middle values for even n */
+  double median;    /* median(x), mean of the two middle values for even n; a NaN ranks as -0, or
+                       below all with its sign bit set, whatever the lengths of the other series */
   double std;       /* population std of the x > 0 */
   double far;       /* (maxsn - median) / std */
   double pssn;      /* (top peak - medc) / stdc; +inf when npeaks <= ntop */

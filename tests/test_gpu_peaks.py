@@ -130,3 +130,22 @@ def test_states_at_word_edges(cuda, n):
             st, idx, val = api.peakstat(torch.from_numpy(x).to(cuda), torch.zeros(1, dtype=torch.int64, device=cuda),
                                         torch.full((1,), n, dtype=torch.int32, device=cuda), 1, n, mpd, 3, 16)
             _check(api.stats_to_numpy(st)[0], idx.cpu().numpy()[0], val.cpu().numpy()[0], x, mpd, 3, 16)
+
+
+@pytest.mark.parametrize("bits", [0x7fc00000, 0x7fffffff, 0x7f800001, 0xffc00000, 0xffffffff])
+@pytest.mark.parametrize("n,count,shift", [(4097, 3, 0.5), (4096, 3, -0.5), (4097, 2500, -0.5), (4096, 2500, 0.5)])
+def test_median_of_a_series_with_nan(cuda, bits, n, count, shift):
+    """A NaN ranks as -0 (sign bit clear) or below all (set) in the median, by itself or beside a longer series,
+    which takes another kernel."""
+    rng = np.random.default_rng(n + count)
+    x = (rng.normal(size=n) + shift).astype(np.float32)
+    x.view(np.uint32)[rng.choice(n, count, replace=False)] = bits
+    ranked = np.sort(np.where(np.isnan(x), np.float32(-np.inf if bits >> 31 else -0.0), x)).astype(np.float64)
+    ref = 0.5 * (ranked[(n - 1) // 2] + ranked[n // 2])
+    for xs in ([x], [x, np.zeros(60000, np.float32)]):
+        lens = np.array([a.size for a in xs])
+        st, _, _ = api.peakstat(torch.from_numpy(np.concatenate(xs)).to(cuda),
+                                torch.from_numpy(np.cumsum(lens) - lens).to(cuda),
+                                torch.from_numpy(lens.astype(np.int32)).to(cuda), 1, int(lens.max()), 10, 4, 8)
+        got = api.stats_to_numpy(st)[0]["median"]
+        assert np.isnan(got) if np.isinf(ref) else got == ref, (len(xs), got, ref)
