@@ -376,10 +376,11 @@ __device__ __forceinline__ float ll2float_fast(long long x) {
 
 constexpr int kSeedStride = 4;  // starts seeded per frequency: every fourth
 
-// The largest value of a warp's lanes (no NaN), in one instruction.
+// The largest value of a warp's lanes (no NaN), in one instruction.  Volatile: every lane must reach it, so
+// it may not follow its result into a lane's own branch.
 __device__ __forceinline__ float warp_max(float v) {
   float r;
-  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return r;
 }
 
