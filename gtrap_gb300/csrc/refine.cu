@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
         cmax = max(cmax, C[b]);
       }
       if (__any_sync(0xffffffffu, cmax > kFineMax)) {   // rare: this trial's sums again, 64 bits at a time
+        __syncwarp();   // (a vote orders no memory: every lane's run has been read and written)
         for (uint32_t b = lane; b < E; b += 32) H[b] = 0;
         __syncwarp();
         for (uint32_t i = lane; i < cv.n; i += 32) {

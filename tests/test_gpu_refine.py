@@ -230,3 +230,23 @@ def test_refine_fine_bins_per_bin(cuda, fine):
     for q in range(2):
         _check(recs[q], OR.refine_curve(tu[:, q], resid[:, q], off[q], ntrue[q], sr[q], p1[q], p2[q], g["fmin"],
                                         g["df"], g["nb"], g["kma"], g["kmi"], g["kkmi"], K=16, S=fine, M=4))
+
+
+@pytest.mark.parametrize("n,phases", [(40000, 16), (70000, 16), (50000, 3)])
+def test_refine_refolds_runs_of_many_bins(cuda, n, phases):
+    """Fine bins past what the 32-bit words hold in a neighbourhood of about a thousand fine bins: the lanes' runs
+    of bins are read before other lanes clear them for the second fold.  The oracle's record, every time."""
+    rng = np.random.default_rng(n)
+    period = 0.5
+    t = (np.arange(n) * np.float32(period / phases)).astype(np.float32)
+    x = rng.normal(0.0, 1e-3, n).astype(np.float32)
+    x[::phases] -= 2e-3
+    nf, fmin, df = 24, np.float32(0.9 / period), np.float32(0.2 / period / 24)
+    g = dict(nf=nf, nb=512, kma=51, kmi=1, kkmi=5, fmin=float(fmin), df=float(df))
+    off, ntrue = np.zeros(3, np.float32), np.full(3, n, np.uint32)
+    sr, p1, p2, recs = _search_and_refine(np.tile(x[:, None], (1, 3)), np.tile(t[:, None], (1, 3)), ntrue, off, g, cuda)
+    o = OR.refine_curve(t, x, off[0], n, sr[0], p1[0], p2[0], g["fmin"], g["df"], g["nb"], g["kma"], g["kmi"], g["kkmi"],
+                        K=KR, S=SR_, M=MR)
+    for q in range(3):
+        _check(recs[q], o)
+        assert recs[q].tobytes() == recs[0].tobytes()
