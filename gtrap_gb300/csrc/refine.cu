@@ -412,10 +412,13 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
       }
     }
     __syncwarp();
-    // the coarse entries as floats (real flux units) and their largest magnitude
+    // the coarse entries as floats and their largest magnitude.  Quantised units: |H| < 2^63 whole numbers,
+    // so a square stays below 2^126, and a power that is not zero above 2^-62: nothing leaves the normal
+    // range (in real units the threshold of a long curve of 2^-50 flux is subnormal, and a bound
+    // multiplied out of it passes over the best window)
     float pm = 0.0f;
     for (int e = lane; e <= iL; e += 32) {
-      const float v = ldexpf(__ll2float_rn(H[e * S]), -sx);
+      const float v = __ll2float_rn(H[e * S]);
       P[e] = make_float2(v, (float)C[e * S]);
       pm = fmaxf(pm, fabsf(v));
     }
@@ -424,7 +427,7 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
     // |P - exact| <= 2^-24 |exact| per entry, so a difference is off by at most 2^-23 pmax
     // plus 2^-24 of itself (both taken twice here); den is exact to 2^-24 and the quotient
     // from __fdividef within 2 ulp, inside the 2^-20 factors
-    const float e0 = ldexpf(pm, -22);
+    const float e0 = pm * (1.0f / 4194304.0f);
     auto power = [&](int ws, int we, double &pw) -> bool {
       const int kk = C[we] - C[ws];
       if (kk <= kkmi) return false;
@@ -439,9 +442,8 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
       const float sv = fabsf(B.x - A.x), hi = sv + (e0 + sv * (1.0f / 4194304.0f));
       return kk > kkmi_f && den > 0.0f ? __fdividef(hi * hi, den) * (1.0f + 1.0f / 1048576.0f) : 0.0f;
     };
-    // (a float prefix near the underflow range would break the bounds: no screening there)
     float thr = 0.0f;
-    if (sx < 100) {
+    {
       // a lower bound of the largest power: first from the windows around the grid's, then raised by every
       // window whose upper bound reaches it; the rows with such a window are the only ones compared
       // exactly.  One product compared a window instead of a quotient: this stage of 64 curves x 65
@@ -488,13 +490,13 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
       }
     };
     for (int s0 = 0; s0 < iL; s0 += 32) {
-      const bool in = s0 + lane < iL && (sx >= 100 || R[s0 + lane] > 0.0f);
+      const bool in = s0 + lane < iL && R[s0 + lane] > 0.0f;
       for (unsigned rows = __ballot_sync(0xffffffffu, in); rows; rows &= rows - 1) {
         const int s = s0 + __ffs(rows) - 1;
         const float2 A = P[s];
         const int wmax = min(kma, iL - s);
         for (int w = kmi + 1 + lane; w <= wmax; w += 32) {
-          if (sx < 100 && upper(A, P[s + w]) < thr) continue;
+          if (upper(A, P[s + w]) < thr) continue;
           const uint32_t ws = s * S, we = (s + w) * S;
           double pw;
           if (power((int)ws, (int)we, pw) && better(pw, ws, we, bp, ba, bb)) { bp = pw; ba = ws; bb = we; }

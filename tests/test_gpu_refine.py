@@ -250,3 +250,31 @@ def test_refine_refolds_runs_of_many_bins(cuda, n, phases):
     for q in range(3):
         _check(recs[q], o)
         assert recs[q].tobytes() == recs[0].tobytes()
+
+
+@pytest.mark.parametrize("exponent", [-110, -56, -51, -50, -49, -48, -40, 60, 100])
+def test_refine_scales_with_the_flux(cuda, exponent):
+    """Flux times a power of two, down to powers below the smallest normal float and up to squares beyond the
+    largest: the same trial and window, SR and depth times the same power of two (noise alone, so that the best
+    power is as small as it gets)."""
+    n, nq, nf, nb, kma, kmi, kkmi = 1 << 18, 8, 64, 2048, 205, 1, 5
+    rng = np.random.default_rng(5)
+    t = np.tile(((np.arange(n) + 0.5) * np.float32(0.0204)).astype(np.float32)[:, None], (1, nq))
+    x = np.ldexp(np.rint(np.ldexp(rng.normal(0, 2.0 ** -11, (n, nq)), 33)), -33).astype(np.float32)
+    span = n * 0.0204
+    fmin, df = float(np.float32(2 / span)), float(np.float32(0.3 / span))
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    T, o, nt = d(t), torch.zeros(nq, device=cuda), torch.full((nq,), n, dtype=torch.int32, device=cuda)
+    sr, p1, p2 = api.geebls(d(x), T, o, nt, nf, nb, kma, kmi, kkmi, fmin, df)
+
+    def refined(flux):
+        return api.refined_to_numpy(api.bls_refine(sr, p1, p2, d(flux), T, o, nt, nb, kma, kmi, kkmi, fmin, df,
+                                                   K=KR, S=SR_, M=MR))
+
+    scaled = np.ldexp(x, exponent).astype(np.float32)
+    assert np.array_equal(np.ldexp(scaled.astype(np.float64), -exponent), x)   # nothing rounded
+    ref, got = refined(x), refined(scaled)
+    for key in ("dk", "kk", "freq", "phase", "duration", "t0"):
+        np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
+    for key in ("sr", "depth"):
+        np.testing.assert_array_equal(got[key], np.ldexp(ref[key], exponent), err_msg=key)
