@@ -5,43 +5,38 @@
 
 #include "common.cuh"
 #include "medgroup.cuh"
-#include "medwindow.cuh"
 
 namespace {
 
-// Groups of T windows (medgroup.cuh).  kGroupMaxR bounds the window of the element-by-element
-// path below, which takes the groups that hold a value that is not finite: the order that a
-// window with NaN is left in is that of the insertion sort and the slides, from the group's
-// first row on.
-using gtrap::kGroupMaxR;
-
-template <int T, class Row>
-__device__ __noinline__ void group_medians_by_slides(int r, Row row, float (&med)[T]) {
-  float win[2 * kGroupMaxR + 1];
-  const int w = 2 * r + 1;
-  bool nan_seen = false;
-  for (int k = 0; k < w; ++k) {
-    win[k] = row(k - r);
-    nan_seen |= isnan(win[k]);
-  }
-  gtrap::window_sort<1>(win, w, nan_seen);
-  for (int k = 0; k < T; ++k) {
-    med[k] = win[r];
-    if (k + 1 == T) break;
-    const float vold = row(k - r), vnew = row(k + 1 + r);
-    if (vnew == vold) continue;
-    nan_seen |= isnan(vnew);
-    gtrap::window_slide<1>(win, w, vold, vnew, nan_seen);
-  }
+// Where row j of a block, from a whole number of groups on, lies: one word of padding a group of T rows.
+template <int T>
+__device__ __forceinline__ int group_slot(int j) {
+  static_assert(T == 4 || T == 8 || T == 16, "groups of 4, 8 or 16 rows");
+  return j + (j >> (T == 16 ? 4 : T == 8 ? 3 : 2));
 }
 
-template <int T, int A, class Row>
-__device__ __forceinline__ void medians_of_group(int r, Row row, float (&med)[T]) {
+// Groups of T windows (medgroup.cuh).  A group that holds a value that is not finite takes the same
+// networks over integer keys, which put NaN in a place of its own.  65,536 x 128, without / with such a value
+// in most groups: r = 5 46 / 69 us, r = 24 81 / 156, r = 63 151 / 290 (by an insertion sort and slides in
+// thread-local memory, which this replaces: 278, 1705, 15,660 us).  A function of its own, taking the
+// pointer: inlined, or with the row accessor passed on, it takes registers from the common path.
+template <int T, int A, int LC>
+__device__ __noinline__ void group_medians_by_keys(const float *mine, int B, float (&med)[T]) {
+  int key[T];
+  float unused = 0.0f;
+  gtrap::group_medians<T, A>(B, [mine](int k) { return gtrap::median_key(mine[group_slot<T>(k) * LC]); }, key, unused);
+#pragma unroll
+  for (int k = 0; k < T; ++k) med[k] = gtrap::median_value(key[k]);
+}
+
+// The medians of the group whose row k lies at mine[group_slot(k) LC].
+template <int T, int A, int LC>
+__device__ __forceinline__ void medians_of_group(const float *mine, int r, float (&med)[T]) {
   float bad = 0.0f;
-  gtrap::group_medians<T, A>(r - T * A, row, med, bad);
+  gtrap::group_medians<T, A>(r - T * A, [mine](int k) { return mine[group_slot<T>(k) * LC]; }, med, bad);
   if (bad != 0.0f) {  // NaN: some value is not finite
     float m[T];
-    group_medians_by_slides<T>(r, row, m);
+    group_medians_by_keys<T, A, LC>(mine, r - T * A, m);
 #pragma unroll
     for (int k = 0; k < T; ++k) med[k] = m[k];
   }
@@ -59,10 +54,8 @@ __global__ void __launch_bounds__(kGroupThreads, T == 16 && A > 1 ? 2 : 3) gfilt
     const float *__restrict__ in, float *__restrict__ out, const unsigned long long *__restrict__ offs,
     const uint32_t *__restrict__ lens, unsigned ncurves, unsigned n_all, int r) {
   extern __shared__ float stage[];
-  constexpr int kLogT = T == 16 ? 4 : T == 8 ? 3 : 2;
-  static_assert((1 << kLogT) == T, "groups of 4, 8 or 16 rows");
   constexpr int kHalo = T * (A + 1);   // > r, a whole number of groups
-  auto slot = [](int j) { return j + (j >> kLogT); };
+  auto slot = [](int j) { return group_slot<T>(j); };
   const int lane = (int)threadIdx.x % LC, group = (int)threadIdx.x / LC, step = (int)blockDim.x / LC;
   const int rows = step * T;
   for (unsigned long long c0 = (unsigned long long)blockIdx.y * LC; c0 < ncurves;
@@ -95,10 +88,9 @@ __global__ void __launch_bounds__(kGroupThreads, T == 16 && A > 1 ? 2 : 3) gfilt
 #pragma unroll
     for (int k = 0; k < T; ++k) res[k] = 0.0f;
     if (live && i0 < n) {
-      auto row = [&](int k) { return mine[slot(k) * LC]; };
-      medians_of_group<T, A>(r, row, res);
+      medians_of_group<T, A, LC>(mine, r, res);
 #pragma unroll
-      for (int k = 0; k < T; ++k) res[k] = __fsub_rn(row(k), res[k]);
+      for (int k = 0; k < T; ++k) res[k] = __fsub_rn(mine[slot(k) * LC], res[k]);
     }
     if constexpr (LC == 32) {
       if (live) {

@@ -7,8 +7,8 @@
 // a network, and one pass over the core copies it, leaving out the former and putting in the
 // latter: 2r + 2 steps for 16 rows, each one element per lane, with the next elements already loaded.
 // The pass writes 16 slots below (ascending) or above (descending, the next time) where it reads, so
-// that the core moves within 16 spare slots.  Values are integer keys in the order of the floats (-0
-// below +0, NaN past the infinities), so that every element that leaves is found, whatever it is.
+// that the core moves within 16 spare slots.  Values are integer keys in the order of the floats
+// (median_key), so that every element that leaves is found, whatever it is.
 //
 // Bound by the latency of the pass's steps at the few warps an SM has room for (five at r = 128), and
 // then by issue.  The first core of a run costs about r / 17 passes, so each lane's run is as long
@@ -21,8 +21,6 @@
 #include "common.cuh"
 #include "medgroup.cuh"
 
-#include <climits>
-
 namespace {
 
 constexpr int kT = 16;
@@ -30,11 +28,8 @@ constexpr int kT = 16;
 constexpr int kE = 2, kL = kE + kT + 1, kS = kL + kT + 1;
 constexpr int kExtraRows = kS + kT + 2;
 
-__device__ __forceinline__ int key_of(float v) {
-  const int b = __float_as_int(v);
-  return max(min(b ^ ((b >> 31) & 0x7fffffff), INT_MAX - 1), INT_MIN + 1);   // INT_MAX and INT_MIN are guards
-}
-__device__ __forceinline__ float value_of(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+using gtrap::median_key;
+using gtrap::median_value;
 
 // One pass: the lane's array at s, in the direction's order, without the kT keys of L (kLeave) and with
 // the kT keys of E, to o.  steps: elements at s + kT.  A step takes the next of E, copies the next
@@ -104,7 +99,7 @@ __global__ void __launch_bounds__(32) gfilter_merge_kernel(const float *__restri
       for (int j = 0; j < kT; ++j) v[j] = row(i + j);
       __syncwarp();   // the loads in flight together
 #pragma unroll
-      for (int j = 0; j < kT; ++j) k[j] = key_of(v[j]);
+      for (int j = 0; j < kT; ++j) k[j] = median_key(v[j]);
     };
     auto put_sorted = [&](int to, const int (&k)[kT]) {
       int s[kT];
@@ -153,7 +148,7 @@ __global__ void __launch_bounds__(32) gfilter_merge_kernel(const float *__restri
 #pragma unroll
       for (int j = 0; j < kT; ++j) {
         const long long i = i0 + j;
-        if (i < n) out[base + (size_t)i * stride] = __fsub_rn(__ldg(x + (size_t)i * stride), value_of(med[j]));
+        if (i < n) out[base + (size_t)i * stride] = __fsub_rn(__ldg(x + (size_t)i * stride), median_value(med[j]));
       }
       if (g + 1 == groups) break;
       keys(i0 + kT - 1 - r, left);

@@ -12,12 +12,23 @@
 //     T / 2 of the 3T / 2 values stay, until one value is left for each window: its median.
 // Every step is a compare-exchange of registers, whatever the values: no shared memory, no
 // divergence, no dependence on how far a value travels.  The result is the order statistic
-// itself, so it equals a sorted window's to the bit.  Values must not be NaN (the caller checks).
+// itself, so it equals a sorted window's to the bit.  Floats must not be NaN (the caller checks); keys may
+// be anything.
 #pragma once
+
+#include <climits>
+#include <type_traits>
 
 namespace gtrap {
 
-// The networks sort floats, or integer keys of the same order.
+// The networks sort floats, or integer keys in the order of the floats: -0 below +0, NaN past the infinity
+// of its sign.  INT_MAX and INT_MIN stay free for guards.
+__device__ __forceinline__ int median_key(float v) {
+  const int b = __float_as_int(v);
+  return max(min(b ^ ((b >> 31) & 0x7fffffff), INT_MAX - 1), INT_MIN + 1);
+}
+__device__ __forceinline__ float median_value(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
 __device__ __forceinline__ float lesser(float a, float b) { return fminf(a, b); }
 __device__ __forceinline__ float greater(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ int lesser(int a, int b) { return min(a, b); }
@@ -59,8 +70,8 @@ __device__ __forceinline__ void net_clean(V (&v)[N]) {
 }
 
 // Two ascending sequences of N into one of 2N.
-template <int N>
-__device__ __forceinline__ void net_merge(const float (&a)[N], const float (&b)[N], float (&out)[2 * N]) {
+template <int N, class V>
+__device__ __forceinline__ void net_merge(const V (&a)[N], const V (&b)[N], V (&out)[2 * N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     out[i] = a[i];
@@ -85,19 +96,19 @@ __device__ __forceinline__ void net_middle(const V (&a)[2 * H], const V (&b)[H],
 
 // The middle N of two ascending sequences of N, ascending (the N / 2 smallest and the N / 2
 // largest left out).
-template <int N>
-__device__ __forceinline__ void net_middle_of_two(const float (&a)[N], const float (&b)[N], float (&out)[N]) {
-  float lo[N], hi[N];   // the N smallest and the N largest, each bitonic
+template <int N, class V>
+__device__ __forceinline__ void net_middle_of_two(const V (&a)[N], const V (&b)[N], V (&out)[N]) {
+  V lo[N], hi[N];   // the N smallest and the N largest, each bitonic
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    lo[i] = fminf(a[i], b[N - 1 - i]);
-    hi[i] = fmaxf(a[i], b[N - 1 - i]);
+    lo[i] = lesser(a[i], b[N - 1 - i]);
+    hi[i] = greater(a[i], b[N - 1 - i]);
   }
-  float u[N / 2], w[N / 2];   // the upper half of the low ones, the lower half of the high ones
+  V u[N / 2], w[N / 2];   // the upper half of the low ones, the lower half of the high ones
 #pragma unroll
   for (int i = 0; i < N / 2; ++i) {
-    u[i] = fmaxf(lo[i], lo[i + N / 2]);
-    w[i] = fminf(hi[i], hi[i + N / 2]);
+    u[i] = greater(lo[i], lo[i + N / 2]);
+    w[i] = lesser(hi[i], hi[i + N / 2]);
   }
   net_clean(u);
   net_clean(w);
@@ -133,52 +144,59 @@ __device__ __forceinline__ void median_halves(const V (&core)[T], const V (&left
 }
 
 // Medians of the windows of rows 0 .. T - 1 (relative to the group), r = T A + B.
-// row(k): the value of row k, -r <= k <= T - 1 + r.  `bad` becomes NaN if a value is not finite
-// (its medians are then not to be used).
-template <int T, int A, class Row>
-__device__ __forceinline__ void group_medians(int B, Row row, float (&med)[T], float &bad) {
+// row(k): the value (V float) or key (V int) of row k, -r <= k <= T - 1 + r.  `bad` becomes NaN if a float
+// is not finite (with a NaN among them the medians are not to be used).
+template <int T, int A, class V, class Row>
+__device__ __forceinline__ void group_medians(int B, Row row, V (&med)[T], float &bad) {
   static_assert(A >= 1 && A <= 3, "cores of one to five whole blocks");
-  auto block = [&](int at, float (&v)[T]) {
+  constexpr bool kFloat = std::is_same<V, float>::value;
+  V least, most;
+  if constexpr (kFloat) { least = -INFINITY; most = INFINITY; }
+  else { least = INT_MIN; most = INT_MAX; }
+  auto check = [&](V v) {
+    if constexpr (kFloat) bad = fmaf(v, 0.0f, bad);
+  };
+  auto block = [&](int at, V (&v)[T]) {
 #pragma unroll
     for (int i = 0; i < T; ++i) {
       v[i] = row(at + i);
-      bad = fmaf(v[i], 0.0f, bad);
+      check(v[i]);
     }
     net_sort(v);
   };
-  float core[T];
+  V core[T];
   {
-    float edge[2 * T];   // the rows on either side of the whole blocks
+    V edge[2 * T];   // the rows on either side of the whole blocks
     {
-      float s[T], p[T];
+      V s[T], p[T];
 #pragma unroll
       for (int i = 0; i < T; ++i) {
         const bool in = i <= B;
-        s[i] = in ? row(-T * A + T - 1 - i) : -INFINITY;
-        p[i] = in ? row(T * A + i) : INFINITY;
-        bad = fmaf(in ? s[i] : 0.0f, 0.0f, bad);
-        bad = fmaf(in ? p[i] : 0.0f, 0.0f, bad);
+        s[i] = in ? row(-T * A + T - 1 - i) : least;
+        p[i] = in ? row(T * A + i) : most;
+        check(in ? s[i] : V(0));
+        check(in ? p[i] : V(0));
       }
       net_sort(s);
       net_sort(p);
       net_merge(s, p, edge);
     }
-    float b0[T];
+    V b0[T];
     if constexpr (A == 1) {
       block(0, b0);
       net_middle<T>(edge, b0, core);
     } else {
-      float pair[2 * T], c[T];
+      V pair[2 * T], c[T];
       block(-T, b0);
       block(T, c);
       net_merge(b0, c, pair);
       if constexpr (A == 2) {   // edge + pair + one block: the middle 2T of the first 4T stay
-        float m[2 * T];
+        V m[2 * T];
         net_middle_of_two<2 * T>(edge, pair, m);
         block(0, b0);
         net_middle<T>(m, b0, core);
       } else {                  // edge + two pairs + one block
-        float all[4 * T], m[2 * T];
+        V all[4 * T], m[2 * T];
         net_merge(edge, pair, all);
         block(-2 * T, b0);
         block(2 * T, c);
@@ -189,15 +207,15 @@ __device__ __forceinline__ void group_medians(int B, Row row, float (&med)[T], f
       }
     }
   }
-  float left[T], right[T];
+  V left[T], right[T];
   const int r = T * A + B;
-  left[0] = right[T - 1] = 0.0f;   // not used
+  left[0] = right[T - 1] = V(0);   // not used
 #pragma unroll
   for (int j = 1; j < T; ++j) {
     left[j] = row(j - 1 - r);
     right[j - 1] = row(r + j);
-    bad = fmaf(left[j], 0.0f, bad);
-    bad = fmaf(right[j - 1], 0.0f, bad);
+    check(left[j]);
+    check(right[j - 1]);
   }
   median_halves<T, T, 0>(core, left, right, med);
 }

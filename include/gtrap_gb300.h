@@ -82,6 +82,8 @@ int gtrap_gather_async(const gtrap_copy *copies, uint32_t count, gtrap_copy *lis
  * against scipy.signal.medfilt(x, 2r+1) followed by a float32 subtraction.
  * Unlike the reference every row is written: n need not be a multiple of a
  * tile height and r is not limited by one.  in and out must not alias.
+ * A NaN in a window ranks past the infinity of its sign for r = 4 .. 888; other radii leave
+ * its rank open.
  * ------------------------------------------------------------------------- */
 int gtrap_gfilter(const float *in, float *out, uint32_t n, uint32_t nq, uint32_t r,
                   gtrap_stream_t stream);

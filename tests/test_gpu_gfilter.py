@@ -181,3 +181,36 @@ def test_gfilter_merged_cores_long_runs(cuda):
     got = api.gfilter(torch.from_numpy(x).to(cuda), 200).cpu().numpy()
     cols = [0, 31, 32, 777, 1499]
     np.testing.assert_array_equal(got[:, cols], oracle.medfilt_residual(np.ascontiguousarray(x[:, cols]), 200))
+
+
+def _median_by_keys(x, r):
+    """x minus the median of its zero-padded windows in the order -NaN, -inf, ..., -0, +0, ..., inf, NaN."""
+    b = x.view(np.int32)
+    key = np.clip(b ^ ((b >> 31) & 0x7fffffff), -2 ** 31 + 1, 2 ** 31 - 2).astype(np.int32)
+    win = np.lib.stride_tricks.sliding_window_view(np.pad(key, ((r, r), (0, 0))), 2 * r + 1, axis=0)
+    med = np.partition(win, r, axis=-1)[..., r]
+    with np.errstate(invalid="ignore"):
+        return x - (med ^ ((med >> 31) & 0x7fffffff)).astype(np.int32).view(np.float32)
+
+
+@pytest.mark.parametrize("r", [4, 7, 8, 15, 16, 24, 31, 32, 47, 48, 63, 64, 65, 128])
+@pytest.mark.parametrize("frac", [0.001, 0.05, 0.6])
+def test_gfilter_windows_with_nan(cuda, r, frac):
+    """NaN of either sign, scattered and as a gap, beside infinities: a window's median is that of the order with
+    NaN past the infinity of its sign, whatever came before the window: image (one, three and 40 curves) and
+    packed."""
+    n = 1300
+    rng = np.random.default_rng(int(1000 * frac) + r)
+    x = rng.normal(1.0, 1e-3, size=(n, 40)).astype(np.float32)
+    x[rng.random(x.shape) < frac] = np.nan
+    x.view(np.uint32)[rng.random(x.shape) < frac / 4] = 0xffc00000
+    x[rng.random(x.shape) < 0.002] = np.inf
+    x[rng.random(x.shape) < 0.002] = -np.inf
+    x[500:700, 1] = np.nan
+    x[:, 2] = rng.normal(size=n)          # a curve without
+    want = _median_by_keys(x, r)
+    for cols in (slice(0, 1), slice(0, 3), slice(0, 40)):
+        got = api.gfilter(torch.from_numpy(np.ascontiguousarray(x[:, cols])).to(cuda), r).cpu().numpy()
+        np.testing.assert_array_equal(got, want[:, cols])
+    for q, got in enumerate(_packed(cuda, [x[:, q].copy() for q in range(5)], r)):
+        np.testing.assert_array_equal(got, want[:, q])
