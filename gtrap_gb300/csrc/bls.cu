@@ -1099,6 +1099,14 @@ int make_plan(uint32_t nb, uint32_t kma, uint32_t nf, uint32_t F_req, Plan *p) {
   return GTRAP_OK;
 }
 
+// Windows hold more than this many bins, at most kma: the kernels index from it as an int.  0 stands for 1
+// (include/geebls.h:26-28), kma and more leave no window.  2^31 and more, a negative number to a caller
+// whose binding wraps it, let every width from one bin on pass, as they always have.
+uint32_t kmi_of(uint32_t kmi, uint32_t kma) {
+  if (kmi >= 1u << 31) return 0;
+  return kmi < 1 ? 1 : kmi < kma ? kmi : kma;
+}
+
 BlsShape shape_of(const Plan &p, uint32_t nb, uint32_t kma, uint32_t kmi_eff, uint32_t kkmi_eff,
                   uint32_t flags) {
   BlsShape sh;
@@ -1147,7 +1155,7 @@ int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const fl
   }
   if (ref_nthread && !exact && kma > ref_nthread)
     return fail(GTRAP_ERR_INVALID_ARG, "%s: reference wrap needs kma <= nthread (%u > %u)", name, kma, ref_nthread);
-  const uint32_t kmi_eff = kmi < 1 ? 1 : kmi;        // include/geebls.h:26-28
+  const uint32_t kmi_eff = kmi_of(kmi, kma);
   const uint32_t kkmi_eff = kkmi < 5 ? 5 : kkmi;     // MINBIN, include/geebls.h:31-33
   const uint32_t n_eff = ref_nthread ? (n / ref_nthread) * ref_nthread : n;  // include/geebls.h:57
 
@@ -1329,7 +1337,7 @@ int gtrap_bls_run(const gtrap_bls_curve *curves, const gtrap_bls_segment *segs, 
   GTRAP_TRY(pool_carve(const_cast<void *>(pool), pool_bytes, total_samples, flags, &X, &AB));
   Plan p;
   GTRAP_TRY(make_plan(nb, kma, 0, F, &p));
-  const uint32_t kmi_eff = kmi < 1 ? 1 : kmi;
+  const uint32_t kmi_eff = kmi_of(kmi, kma);
   const BlsShape sh = shape_of(p, nb, kma, kmi_eff, 5, flags);
   BlsQueue qa;
   qa.curves = curves; qa.segs = segs; qa.cum = cum; qa.nseg = nseg;

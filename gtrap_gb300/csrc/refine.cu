@@ -623,6 +623,8 @@ int refine_common(RefArgs &a, uint32_t count, void *workspace, size_t workspace_
   if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < need)
     return fail(GTRAP_ERR_WORKSPACE, "%s: workspace of %zu bytes (256-byte aligned) needed", name, need);
   if (count > 65535u * 4u) return fail(GTRAP_ERR_INVALID_ARG, "%s: at most %u curves per call", name, 65535u * 4u);
+  // more than kmi bins and at most kma: no window from kma on, and the kernels index from kmi as an int
+  a.kmi = a.kmi < 1 ? 1 : a.kmi < a.kma ? a.kmi : a.kma;
   a.lognb = gtrap::ilog2u(a.nb);
   a.logK = gtrap::ilog2u(a.K);
   a.part = reinterpret_cast<Part *>(workspace);
@@ -668,7 +670,7 @@ int gtrap_bls_refine(const float *blsp, const uint32_t *phase1, const uint32_t *
   a.blsp = blsp; a.ph1 = phase1; a.ph2 = phase2; a.t = tu; a.x = lc;
   a.offset = offset; a.ntrue = ntrue;
   a.n = n; a.nq = nq; a.nf = nf; a.kkmi = kkmi; a.fmin = fmin; a.df = df;
-  a.nb = nb; a.kma = kma; a.kmi = kmi < 1 ? 1 : kmi; a.K = K; a.S = S; a.M = M;
+  a.nb = nb; a.kma = kma; a.kmi = kmi; a.K = K; a.S = S; a.M = M;
   a.out = out;
   return refine_common(a, nq, workspace, workspace_bytes, stream, "bls_refine");
 }
@@ -683,7 +685,7 @@ int gtrap_bls_refine_packed(const float *blsp, const uint32_t *phase1, const uin
   RefArgs a = {};
   a.blsp = blsp; a.ph1 = phase1; a.ph2 = phase2; a.t = t; a.x = x;
   a.curves = curves; a.sel = sel;
-  a.nb = nb; a.kma = kma; a.kmi = kmi < 1 ? 1 : kmi; a.K = K; a.S = S; a.M = M;
+  a.nb = nb; a.kma = kma; a.kmi = kmi; a.K = K; a.S = S; a.M = M;
   a.out = out;
   return refine_common(a, count, workspace, workspace_bytes, stream, "bls_refine_packed");
 }

@@ -187,3 +187,27 @@ def test_lone_curve_takes_smaller_blocks(cuda, nf, nb):
     for one, many in zip(run(1), run(nq)):
         assert torch.equal(one[0].view(torch.int32), many[0].view(torch.int32))
         assert torch.equal(one[0].view(torch.int32), many[-1].view(torch.int32))
+
+
+@pytest.mark.parametrize("nb,kma", [(256, 27), (1024, 103)])
+def test_kmi_past_the_range_of_widths(cuda, nb, kma):
+    """kmi from kma on leaves no window; negative numbers, which the binding wraps to 2^31 and more, all pass every
+    width from one bin on (the kernels index from kmi: none of these may reach them)."""
+    n, nf = 1500, 40
+    rng = np.random.default_rng(nb)
+    t = np.tile((np.arange(n) * np.float32(0.0204)).astype(np.float32)[:, None], (1, 2))
+    lc = rng.normal(0, 1e-3, (n, 2)).astype(np.float32)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    T, X, off, nt = d(t), d(lc), torch.zeros(2, device=cuda), torch.full((2,), n, dtype=torch.int32, device=cuda)
+    run = lambda kmi: [v.cpu().numpy() for v in api.geebls(X, T, off, nt, nf, nb, kma, kmi, 5, 0.05, 0.02)]
+    for kmi in (kma, kma + 1, 2 ** 31 - 1):
+        assert not run(kmi)[0].any()
+    one, low = run(1), run(-1)
+    assert np.all(low[0] >= one[0])
+    for kmi in (-2, -40, -100000, -2 ** 31):
+        for a, b in zip(run(kmi), low):
+            np.testing.assert_array_equal(a, b)
+    sr, p1, p2 = (d(v) for v in one)
+    for kmi in (kma, 2 ** 31 - 1, -1, -100000, -2 ** 31):
+        rec = api.refined_to_numpy(api.bls_refine(sr, p1, p2, X, T, off, nt, nb, kma, kmi, 5, 0.05, 0.02, K=8, S=4, M=4))
+        assert not rec["sr"].any() and not rec["kk"].any()
