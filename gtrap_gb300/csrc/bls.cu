@@ -318,7 +318,7 @@ struct BlsShape {
   uint32_t flags;
 };
 
-// One block's work: F consecutive trial frequencies of one curve.
+// One block's work: trial frequencies j0, j0 + js, ... of one curve (js = 1 where not kSpread).
 struct BlsTile {
   const int32_t *X;        // quantised flux of the curve's samples (kMasked = not folded)
   const ulonglong2 *AB;    // exact phase pairs (frac(t*fmin), frac(t*df)) as 64-bit fractions
@@ -327,9 +327,9 @@ struct BlsTile {
   float N;                 // denominator count of the power
   float kkmi;              // windows must hold more than kkmi samples
   int sx, CB;              // flux scale exponent, count bits of the 64-bit format
-  uint32_t j0, nfrem;      // first frequency index, frequencies in this tile
+  uint32_t j0, js, nfrem;  // first frequency index, step to the next, frequencies in this tile
   float fmin, df;          // frequency grid (FP32-reference phase)
-  float *blsp;             // outputs of frequency j0 (nfrem consecutive elements)
+  float *blsp;             // outputs of frequency j0 (nfrem elements js apart)
   uint32_t *ph1, *ph2;
 };
 
@@ -390,7 +390,7 @@ __device__ __forceinline__ void group_bar(int id, int nthreads) {
 
 // Fold + scan of one tile by the whole block (blockDim.x == kThreads).
 // MODE 0: exact phase, nb power of two; 1: exact phase, any nb; 2: FP32 reference phase.
-template <int R, int MODE>
+template <int R, int MODE, bool kSpread>
 __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
   extern __shared__ __align__(16) unsigned long long sm[];
   __shared__ unsigned long long best_key[64];    // per frequency: best (power, -start, -end)
@@ -403,7 +403,7 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
   __shared__ int scan_m[kThreads / 32];          // per-warp maximum bin count
   __shared__ unsigned drop_cnt[64];              // FP32-phase samples landing on bin nb
 
-  const uint32_t j0 = tj.j0;
+  const uint32_t j0 = tj.j0, js = kSpread ? tj.js : 1u;
   const uint32_t nfrem = tj.nfrem;
   const int tid = threadIdx.x;
   const int nb = (int)a.nb;
@@ -434,10 +434,10 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
   const float nbf = (float)nb;
   const bool f0_nofma = a.flags & GTRAP_BLS_REF_F0_NOFMA;
   const bool ph_fma = a.flags & GTRAP_BLS_REF_PH_FMA;
-  // bin of time t at frequency j0 + f with the reference's float32 arithmetic; nb means
+  // bin of time t at the tile's frequency f with the reference's float32 arithmetic; nb means
   // dropped (the reference's wrap overwrites that slot)
   auto ref_bin = [&](float t, uint32_t f) -> uint32_t {
-    const float jf = (float)(j0 + f);
+    const float jf = (float)(j0 + f * js);
     const float f0 = f0_nofma ? __fadd_rn(tj.fmin, __fmul_rn(tj.df, jf)) : __fmaf_rn(tj.df, jf, tj.fmin);
     const float p = __fmul_rn(t, f0);
     const float ip = __int2float_rn(__float2int_rz(p));
@@ -465,11 +465,12 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
           const unsigned wS = (unsigned)(xq[u] >> 10);
           const unsigned wC = ((unsigned)(xq[u] & 1023) << 12) | 1u;
           unsigned long long ph = ab[u].x + (unsigned long long)j0 * ab[u].y;
+          const unsigned long long step = kSpread ? js * ab[u].y : ab[u].y;
           auto add = [&](unsigned *h) {
             const uint32_t bin = MODE == 0 ? (uint32_t)(ph >> shift) : (uint32_t)__umul64hi(ph, (unsigned long long)nb);
             atomicAdd(h + bin, wS);
             atomicAdd(h + nbp + bin, wC);
-            ph += ab[u].y;
+            ph += step;
           };
           if constexpr (NF > 0) {
 #pragma unroll
@@ -511,7 +512,7 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
       }
     }
   }
-  // 64-bit re-fold of frequency j0 + f by the Tg_ threads of one group
+  // 64-bit re-fold of the tile's frequency f by the Tg_ threads of one group
   auto refold64 = [&](uint32_t f, int gtid_, int Tg_) {
     unsigned long long *Hf = sm + (size_t)f * a.region;
     for (uint32_t k = gtid_; k < tj.n; k += Tg_) {
@@ -521,7 +522,7 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
       uint32_t bin;
       if (MODE != 2) {
         const ulonglong2 ab = ABq[k];
-        const unsigned long long ph = ab.x + (unsigned long long)(j0 + f) * ab.y;
+        const unsigned long long ph = ab.x + (unsigned long long)(j0 + f * js) * ab.y;
         bin = MODE == 0 ? (uint32_t)(ph >> shift) : (uint32_t)__umul64hi(ph, (unsigned long long)nb);
       } else {
         bin = ref_bin(__ldg(Tq + k), f);
@@ -925,14 +926,16 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
     const bool found = key != 0ull;
     const float pw = __uint_as_float((unsigned)(key >> 32));
     const unsigned ie = 0xffffffffu - (unsigned)(key & 0xffffffffull);
-    tj.blsp[tid] = found ? ldexpf(sqrtf(pw), -tj.sx) : 0.0f;
-    if (tj.ph1) tj.ph1[tid] = found ? (ie >> 15) : 0u;
-    if (tj.ph2) tj.ph2[tid] = found ? (ie & 0x7fffu) - 1u : 0u;
+    const uint32_t o = (uint32_t)tid * js;
+    tj.blsp[o] = found ? ldexpf(sqrtf(pw), -tj.sx) : 0.0f;
+    if (tj.ph1) tj.ph1[o] = found ? (ie >> 15) : 0u;
+    if (tj.ph2) tj.ph2[o] = found ? (ie & 0x7fffu) - 1u : 0u;
   }
 }
 
-// Plain launch: one block per (curve, tile) of an [n, nq] image batch.
-template <int R, int MODE>
+// Plain launch: one block per (curve, tile) of an [n, nq] image batch.  A tile takes F consecutive
+// frequencies or, with kSpread, every tiles-th one (see spread_tiles).
+template <int R, int MODE, bool kSpread>
 __global__ void __launch_bounds__(kThreads, R == 8 ? kMinBlocks : 1)
 bls_fold_scan_kernel(const BlsShape sh, const BlsArgs a) {
   // the tile descriptor lives in shared memory: read where used, not held in registers
@@ -950,8 +953,9 @@ bls_fold_scan_kernel(const BlsShape sh, const BlsArgs a) {
   t.kkmi = (float)sh.kkmi;
   t.sx = a.sx[q];
   t.CB = a.CB;
-  t.j0 = tile * sh.F;
-  t.nfrem = min(sh.F, a.nf - t.j0);
+  t.j0 = kSpread ? tile : tile * sh.F;
+  t.js = kSpread ? a.tiles : 1u;
+  t.nfrem = kSpread ? (a.nf - tile + a.tiles - 1) / a.tiles : min(sh.F, a.nf - t.j0);
   t.fmin = a.fmin;
   t.df = a.df;
   const size_t o = (size_t)q * a.nf + t.j0;
@@ -960,7 +964,7 @@ bls_fold_scan_kernel(const BlsShape sh, const BlsArgs a) {
   t.ph2 = a.ph2 ? a.ph2 + o : nullptr;
   }
   __syncthreads();
-  bls_tile<R, MODE>(sh, t);
+  bls_tile<R, MODE, kSpread>(sh, t);
 }
 
 // Persistent launch over a device work queue of (curve, tile) items of a packed batch.
@@ -977,7 +981,7 @@ struct BlsQueue {
   uint32_t *counter;       // next item (zeroed before the launch)
 };
 
-template <int R, int MODE>
+template <int R, int MODE, bool kSpread>
 __global__ void __launch_bounds__(kThreads, R == 8 ? kMinBlocks : 1)
 bls_queue_kernel(const BlsShape sh, const BlsQueue qa) {
   __shared__ uint32_t item_s;
@@ -996,8 +1000,12 @@ bls_queue_kernel(const BlsShape sh, const BlsQueue qa) {
     }
     const gtrap_bls_segment sg = qa.segs[lo];
     const gtrap_bls_curve c = qa.curves[sg.curve];
-    const uint32_t j0 = (sg.tile0 + (it - qa.cum[lo])) * sh.F;
-    if (j0 >= c.nf) continue;  // uniform across the block
+    // kSpread: where the segment is a whole curve, its tiles take every tiles-th frequency (spread_tiles);
+    // the tiles of a part of one take consecutive frequencies, so that a tile's number tells which
+    const uint32_t tiles = (c.nf + sh.F - 1) / sh.F, tile = sg.tile0 + (it - qa.cum[lo]);
+    if (tile >= tiles) continue;  // uniform across the block
+    const bool spread = kSpread && sg.tile0 == 0 && qa.cum[lo + 1] - qa.cum[lo] >= tiles;
+    const uint32_t j0 = spread ? tile : tile * sh.F;
     if (threadIdx.x == 0) {
     t.X = qa.X + c.off;
     t.AB = qa.AB ? qa.AB + c.off : nullptr;
@@ -1009,7 +1017,8 @@ bls_queue_kernel(const BlsShape sh, const BlsQueue qa) {
     t.sx = c.sx;
     t.CB = c.cb;
     t.j0 = j0;
-    t.nfrem = min(sh.F, c.nf - j0);
+    t.js = spread ? tiles : 1u;
+    t.nfrem = spread ? (c.nf - tile + tiles - 1) / tiles : min(sh.F, c.nf - j0);
     t.fmin = c.fmin;
     t.df = c.df;
     t.blsp = qa.blsp + c.out + j0;
@@ -1017,7 +1026,7 @@ bls_queue_kernel(const BlsShape sh, const BlsQueue qa) {
     t.ph2 = qa.ph2 ? qa.ph2 + c.out + j0 : nullptr;
     }
     __syncthreads();
-    bls_tile<R, MODE>(sh, t);
+    bls_tile<R, MODE, kSpread>(sh, t);
   }
 }
 
@@ -1043,9 +1052,13 @@ size_t bls_static_smem() {
   }
   const uint32_t c = cached[dev].load(std::memory_order_relaxed);
   if (c) return c - 1;
-  const void *fns[] = {(const void *)bls_fold_scan_kernel<8, 0>, (const void *)bls_fold_scan_kernel<8, 1>,
-                       (const void *)bls_fold_scan_kernel<8, 2>, (const void *)bls_queue_kernel<8, 0>,
-                       (const void *)bls_queue_kernel<8, 1>, (const void *)bls_queue_kernel<8, 2>};
+  const void *fns[] = {
+      (const void *)bls_fold_scan_kernel<8, 0, false>, (const void *)bls_fold_scan_kernel<8, 1, false>,
+      (const void *)bls_fold_scan_kernel<8, 2, false>, (const void *)bls_fold_scan_kernel<8, 0, true>,
+      (const void *)bls_fold_scan_kernel<8, 1, true>,  (const void *)bls_fold_scan_kernel<8, 2, true>,
+      (const void *)bls_queue_kernel<8, 0, false>,     (const void *)bls_queue_kernel<8, 1, false>,
+      (const void *)bls_queue_kernel<8, 2, false>,     (const void *)bls_queue_kernel<8, 0, true>,
+      (const void *)bls_queue_kernel<8, 1, true>,      (const void *)bls_queue_kernel<8, 2, true>};
   size_t mx = 0;
   for (const void *fn : fns) {
     cudaFuncAttributes fa;
@@ -1136,6 +1149,24 @@ size_t ws_size(uint32_t n, uint32_t nq, uint32_t flags, bool full) {
 // 526 / 536 us).  Blocks of 2 or 3 re-read the samples too often (149 and 143 us in the first case).
 constexpr uint32_t kFewF = 4;
 
+// Whether a launch's tiles take every tiles-th frequency instead of consecutive ones.  At a few
+// frequencies of an evenly sampled curve (a step of about 16, 32, 48 bins from sample to sample) the lanes
+// of a warp meet in one bank, or many samples in one bin, and the fold takes up to twice as long; neighbouring
+// frequencies share that, so a block of consecutive ones is slow as a whole, and the launch waits for it.
+// Consecutive / spread, 65,000 samples at 29.4 min, one curve: 1800 frequencies, nb = 2048 412 / 299 us,
+// nb = 512 464 / 283; five curves, 2048 frequencies, nb = 2048 1238 / 1070; 8 curves of 65,536 and 16,384
+// frequencies 7420 / 7367.  Large launches of short curves (64 x 4096: 4122 / 4174; the step to the next
+// frequency is a product a sample) and of 4096 bins (5 x 65,000, 2048 frequencies 1307 / 1332) lose a little.
+constexpr uint32_t kSpreadMinN = 8192, kSpreadMaxNb = 2048;
+// the same for the segments of a work queue, by their number (their lengths are on the device): one curve of
+// 65,000 samples, 1800 frequencies, nb = 2048 417 / 268 us, twelve of 18,000, 2000 frequencies, nb = 512
+// 846 / 768; a batch of 80 curves of all lengths 10,150 / 10,212
+constexpr uint32_t kSpreadSegments = 16;
+bool spread_tiles(const Plan &p, uint32_t n, uint32_t nq, uint32_t nb) {
+  return (uint64_t)p.tiles * nq <= 2ull * kMinBlocks * gtrap::sm_count() ||
+         (n >= kSpreadMinN && nb <= kSpreadMaxNb);
+}
+
 int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const float *lc,
             const float *tu, const float *offset, const uint32_t *ntrue, uint32_t n, uint32_t nq,
             uint32_t nf, uint32_t nb, uint32_t kma, uint32_t kmi, uint32_t kkmi, float fmin,
@@ -1212,10 +1243,15 @@ int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const fl
   if (blocks >= (1ull << 31)) return fail(GTRAP_ERR_INVALID_ARG, "%s: grid too large", name);
   const void *fn;
   const int mode = !exact ? 2 : (gtrap::is_pow2(nb) ? 0 : 1);
+  const bool spread = spread_tiles(p, n, nq, nb);
 #define GTRAP_BLS_LAUNCH(RR, MM)                                                          \
-  fn = (const void *)bls_fold_scan_kernel<RR, MM>;                                         \
+  fn = spread ? (const void *)bls_fold_scan_kernel<RR, MM, true>                           \
+              : (const void *)bls_fold_scan_kernel<RR, MM, false>;                         \
   GTRAP_TRY(gtrap::ensure_smem(fn, p.smem, name));                                         \
-  bls_fold_scan_kernel<RR, MM><<<(unsigned)blocks, kThreads, p.smem, stream>>>(sh, ba);
+  if (spread)                                                                              \
+    bls_fold_scan_kernel<RR, MM, true><<<(unsigned)blocks, kThreads, p.smem, stream>>>(sh, ba);  \
+  else                                                                                     \
+    bls_fold_scan_kernel<RR, MM, false><<<(unsigned)blocks, kThreads, p.smem, stream>>>(sh, ba);
   if (p.R == 8) {
     if (mode == 0) { GTRAP_BLS_LAUNCH(8, 0) } else if (mode == 1) { GTRAP_BLS_LAUNCH(8, 1) } else { GTRAP_BLS_LAUNCH(8, 2) }
   } else {
@@ -1348,19 +1384,24 @@ int gtrap_bls_run(const gtrap_bls_curve *curves, const gtrap_bls_segment *segs, 
   const int mode = !exact ? 2 : (gtrap::is_pow2(nb) ? 0 : 1);
   const void *fn;
   // blocks == 0: as many as fit on the SMs at once (the queue keeps them busy)
+  const bool spread = nseg <= kSpreadSegments;
 #define GTRAP_BLS_QLAUNCH(RR, MM)                                                          \
-  fn = (const void *)bls_queue_kernel<RR, MM>;                                              \
+  fn = spread ? (const void *)bls_queue_kernel<RR, MM, true>                                \
+              : (const void *)bls_queue_kernel<RR, MM, false>;                              \
   GTRAP_TRY(gtrap::ensure_smem(fn, p.smem, "bls_run"));                                     \
   if (blocks == 0) {                                                                        \
     int per_sm = 0;                                                                         \
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bls_queue_kernel<RR, MM>,    \
-                                                      kThreads, p.smem) != cudaSuccess) {   \
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, p.smem) !=     \
+        cudaSuccess) {                                                                      \
       cudaGetLastError();                                                                   \
       per_sm = 1;                                                                           \
     }                                                                                       \
     blocks = (uint32_t)(gtrap::sm_count() * (per_sm > 0 ? per_sm : 1));                     \
   }                                                                                         \
-  bls_queue_kernel<RR, MM><<<blocks, kThreads, p.smem, stream>>>(sh, qa);
+  if (spread)                                                                               \
+    bls_queue_kernel<RR, MM, true><<<blocks, kThreads, p.smem, stream>>>(sh, qa);           \
+  else                                                                                      \
+    bls_queue_kernel<RR, MM, false><<<blocks, kThreads, p.smem, stream>>>(sh, qa);
   if (p.R == 8) {
     if (mode == 0) { GTRAP_BLS_QLAUNCH(8, 0) } else if (mode == 1) { GTRAP_BLS_QLAUNCH(8, 1) } else { GTRAP_BLS_QLAUNCH(8, 2) }
   } else {

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import oracle
-from gtrap_gb300 import batch as B, synth
+from gtrap_gb300 import api, batch as B, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -205,3 +205,56 @@ def test_tile_plan_keeps_two_blocks_per_sm(cuda):
     # the plan subtracts the kernels' queried static shared memory and the reservation from
     # half an SM: more static bytes would drop F to 5 here
     assert int(N.fn("gtrap_bls_tile_frequencies")(2048, 205)) == 6
+
+
+@pytest.mark.parametrize("nb,nf,phase", [(1024, 1, "exact"), (1024, 5, "exact"), (1024, 131, "exact"), (1000, 64, "exact"),
+                                         (2048, 45, "fp32"), (8192, 13, "exact"), (8192, 7, "fp32"), (64, 200, "exact")])
+def test_spread_and_consecutive_tiles_give_the_same_bits(cuda, nb, nf, phase):
+    """Few segments of whole curves take every tiles-th frequency a tile, many segments and parts of a curve
+    consecutive ones; an image of long curves the former, of short ones in a big launch the latter.  Grids of one
+    frequency, of less than a tile, of whole tiles and of a remainder; nothing but the curve's spectrum written."""
+    rng = np.random.default_rng(nb + nf)
+    n = 8200
+    t = np.sort(rng.uniform(0, 160, n)).astype(np.float32)
+    x = rng.normal(0, 1e-3, n).astype(np.float32)
+    spec = B.BlsSpec(nb=nb, kma=max(2, nb // 10), kmi=1, phase=phase)
+
+    def batch(count):
+        bat = B.RaggedBatch(spec)
+        for _ in range(count):
+            bat.add_bls(t, x, nf, 0.05, 0.004, kkmi=10)
+        bat.build()
+        bat.launch()
+        return bat
+
+    few, many = batch(1), batch(20)
+    ref = [v.copy() for v in few.bls_result(0)]
+    assert ref[0].any()
+    for k in (0, 7, 19):
+        for a, b in zip(ref, many.bls_result(k)):
+            np.testing.assert_array_equal(a, b)
+    # the first tiles alone, and the curve in two segments
+    F = few.F
+    tiles = (nf + F - 1) // F
+    for parts in ([(0, tiles - 1)], [(0, tiles // 2), (tiles // 2, tiles)]):
+        few.blsp.fill_(-1.0)
+        segs = np.zeros(len(parts), B.SEGMENT)
+        segs["tile0"] = [a for a, _ in parts]
+        cum = np.cumsum([0] + [b - a for a, b in parts]).astype(np.uint32)
+        if cum[-1] == 0:
+            continue
+        few.launch_bls(queue=few._upload_segments(segs, cum))
+        got, end = few.bls_result(0)[0], min(nf, F * parts[-1][1])
+        np.testing.assert_array_equal(got[:end], ref[0][:end])
+        assert (got[end:] == -1.0).all()
+    # the image forms: one curve, and enough of them to fill the GPU several times
+    img = [np.ascontiguousarray(v)[:, None] for v in (x, t)]
+    d = lambda a, k: torch.from_numpy(a).to(cuda).expand(n, k).contiguous()
+    off = float(np.frombuffer(few.bls_curves.cpu().numpy().tobytes(), B.BLS_CURVE)[0]["offset"])
+    for k in (1, 40 if nb >= 1000 else 3):
+        sr, p1, p2 = api.geebls(d(img[0], k), d(img[1], k), torch.full((k,), off, device=cuda),
+                                torch.full((k,), n, dtype=torch.int32, device=cuda), nf, nb, spec.kma, 1, 10, 0.05,
+                                0.004, phase=phase)
+        for a, b in zip(ref, (sr, p1, p2)):
+            for q in (0, k - 1):
+                np.testing.assert_array_equal(a, b[q].cpu().numpy().view(a.dtype))
