@@ -1154,17 +1154,18 @@ constexpr uint32_t kFewF = 4;
 // of a warp meet in one bank, or many samples in one bin, and the fold takes up to twice as long; neighbouring
 // frequencies share that, so a block of consecutive ones is slow as a whole, and the launch waits for it.
 // Consecutive / spread, 65,000 samples at 29.4 min, one curve: 1800 frequencies, nb = 2048 412 / 299 us,
-// nb = 512 464 / 283; five curves, 2048 frequencies, nb = 2048 1238 / 1070; 8 curves of 65,536 and 16,384
-// frequencies 7420 / 7367.  Large launches of short curves (64 x 4096: 4122 / 4174; the step to the next
-// frequency is a product a sample) and of 4096 bins (5 x 65,000, 2048 frequencies 1307 / 1332) lose a little.
-constexpr uint32_t kSpreadMinN = 8192, kSpreadMaxNb = 2048;
+// nb = 512 464 / 283, 3000 frequencies, nb = 256 600 / 404; five curves, 2048 frequencies, nb = 2048
+// 1238 / 1070; 8 curves of 65,536 and 16,384 frequencies 7420 / 7340.  Not for short curves (64 x 4096, 4096
+// frequencies: 4122 / 4174; the step to the next frequency is a product a sample), not for 4096 bins, whose steps
+// pass many such places (2 x 40,000, 400 frequencies: 132 / 188), and not for few bins, where some
+// frequencies are folded again in 64 bits, best several in a block at once (2 x 40,000, nb = 100: 715 / 865).
+constexpr uint32_t kSpreadMinN = 8192, kSpreadMinNb = 256, kSpreadMaxNb = 2048;
 // the same for the segments of a work queue, by their number (their lengths are on the device): one curve of
 // 65,000 samples, 1800 frequencies, nb = 2048 417 / 268 us, twelve of 18,000, 2000 frequencies, nb = 512
 // 846 / 768; a batch of 80 curves of all lengths 10,150 / 10,212
 constexpr uint32_t kSpreadSegments = 16;
-bool spread_tiles(const Plan &p, uint32_t n, uint32_t nq, uint32_t nb) {
-  return (uint64_t)p.tiles * nq <= 2ull * kMinBlocks * gtrap::sm_count() ||
-         (n >= kSpreadMinN && nb <= kSpreadMaxNb);
+bool spread_tiles(uint32_t n, uint32_t nb) {
+  return n >= kSpreadMinN && nb >= kSpreadMinNb && nb <= kSpreadMaxNb;
 }
 
 int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const float *lc,
@@ -1243,7 +1244,7 @@ int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const fl
   if (blocks >= (1ull << 31)) return fail(GTRAP_ERR_INVALID_ARG, "%s: grid too large", name);
   const void *fn;
   const int mode = !exact ? 2 : (gtrap::is_pow2(nb) ? 0 : 1);
-  const bool spread = spread_tiles(p, n, nq, nb);
+  const bool spread = spread_tiles(n, nb);
 #define GTRAP_BLS_LAUNCH(RR, MM)                                                          \
   fn = spread ? (const void *)bls_fold_scan_kernel<RR, MM, true>                           \
               : (const void *)bls_fold_scan_kernel<RR, MM, false>;                         \
@@ -1384,7 +1385,7 @@ int gtrap_bls_run(const gtrap_bls_curve *curves, const gtrap_bls_segment *segs, 
   const int mode = !exact ? 2 : (gtrap::is_pow2(nb) ? 0 : 1);
   const void *fn;
   // blocks == 0: as many as fit on the SMs at once (the queue keeps them busy)
-  const bool spread = nseg <= kSpreadSegments;
+  const bool spread = nseg <= kSpreadSegments && nb >= kSpreadMinNb && nb <= kSpreadMaxNb;
 #define GTRAP_BLS_QLAUNCH(RR, MM)                                                          \
   fn = spread ? (const void *)bls_queue_kernel<RR, MM, true>                                \
               : (const void *)bls_queue_kernel<RR, MM, false>;                              \

@@ -156,7 +156,8 @@ int gtrap_geebls_simple(float *blsp, uint32_t *phase1, uint32_t *phase2, const f
  * Curve q owns samples [off, off + n) of the packed time/flux arrays and output elements
  * [out, out + nf) of the packed spectra.  A segment asks for tiles [tile0, tile0 + count) of
  * one curve, tile t covering frequencies [t*F, min((t+1)*F, nf)); cum[k] is the number of
- * tiles of segments 0..k-1 (cum[nseg] = total).  All arrays are device memory, so a batch
+ * tiles of segments 0..k-1 (cum[nseg] = total).  (A segment of all of a curve's tiles may share
+ * the same frequencies out over them otherwise.)  All arrays are device memory, so a batch
  * can be captured in a CUDA graph and replayed.
  * ------------------------------------------------------------------------- */
 typedef struct {
