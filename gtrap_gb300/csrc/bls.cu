@@ -30,6 +30,7 @@
 //    lowest-(start, end) tie-break.  Every bound is conservative under float rounding, so the
 //    outputs equal an exhaustive scan of the same prefix arrays.
 #include <atomic>
+#include <cfloat>
 #include <type_traits>
 
 #include "common.cuh"
@@ -374,6 +375,13 @@ __device__ __forceinline__ float ll2float_fast(long long x) {
   return __fmaf_rn(__int2float_rn(h), 4294967296.0f, __int2float_rn(l));
 }
 
+// A unit with more rows and more columns left than kDense bounds its starts in blocks of eight, where windows are
+// of at most kDenseKma bins: a unit's bound pairs its widest windows' flux with its narrowest ones' counts, which
+// is loose where its 31 bins are much of a width, and smooth or strong signals then leave most of it.  200
+// curves of 5000 samples, 1000 frequencies, without / with: slow trends, nb = 1024, kma = 102 18.0 / 11.6 ms; deep
+// transits, nb = 512, kma = 51 6.1 / 3.7 ms; 64 x 4096, kma = 103 4122 / 3875 us.  Wider windows lose by it
+// (nb = 512, kma = 204, trends 4.9 / 6.3 ms).
+constexpr int kDense = 8, kDenseKma = 160;
 constexpr int kSeedStride = 4;  // starts seeded per frequency: every fourth
 
 // The largest value of a warp's lanes (no NaN), in one instruction.  Volatile: every lane must reach it, so
@@ -800,8 +808,9 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
   const int oc0 = (kmi + 1) >> 5;                          // first chunk of ends, from the starts' chunk
   const int nco = max(1, ((31 + kma) >> 5) - oc0 + 1);     // chunks of ends a chunk of starts reaches
   const int nunit = nsc * nco;
-  // units a warp job: half a warp's where the tile has few, so that the jobs spread evenly
-  const int upj = (int)nfrem * nunit < 32 * 6 * (kThreads / 32) ? 16 : 32;
+  // units a warp job: fewer where a frequency or the tile has few, so that the jobs spread evenly
+  // (2 x 40,000, nb = 256, strong transits 618 / 599 us)
+  const int upj = nunit < 64 ? 8 : (int)nfrem * nunit < 32 * 6 * (kThreads / 32) ? 16 : 32;
   const int njob_f = (nunit + upj - 1) / upj;
   const int njob = (kma > kmi) ? (int)nfrem * njob_f : 0;
   // divisions by njob_f and nco as multiply-highs: exact, dividend times divisor < 2^32
@@ -847,7 +856,7 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
       live &= live - 1;
       const int s32 = 32 * __shfl_sync(0xffffffffu, us, src);
       const int e32 = 32 * __shfl_sync(0xffffffffu, uc, src);
-      const float thr = __uint_as_float(best_thr[f]) * kSlack;
+      const float thr = fminf(__uint_as_float(best_thr[f]), FLT_MAX) * kSlack;
       const int e = swz(e32 + lane), i = swz(s32 + lane);   // the lane's end and start
       const bool e_in = e <= elast && e >= s32 + kmi + 1 && e <= s32 + 31 + kma;
       const float2 Pe = e_in ? P[e32 + lane] : make_float2(0.0f, 0.0f);
@@ -883,9 +892,9 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
         const float kk = B.y - A.y;
         const float den = kk * ((Nf + A.y) - B.y);
         const float s2 = s * s;
-        // den <= 0 (a window holding every sample) gives an infinite or negative power
-        if ((unsigned)(ee - ii - kmi - 1) < (unsigned)(kma - kmi) && kk > kkmi_f &&
-            (den <= 0.0f || fmaf(-thr, den, s2) >= 0.0f)) {
+        // den <= 0 (a window holding every sample) gives an infinite or negative power: it passes, the
+        // threshold being finite
+        if ((unsigned)(ee - ii - kmi - 1) < (unsigned)(kma - kmi) && kk > kkmi_f && fmaf(-thr, den, s2) >= 0.0f) {
           const float pw = __fdiv_rn(s2, den);
           const int key = (ii << 15) | ee;
           if (pw > 0.0f && (pw > bpow || (pw == bpow && key < bk))) {
@@ -894,7 +903,33 @@ __device__ __forceinline__ void bls_tile(const BlsShape a, const BlsTile &tj) {
           }
         }
       };
-      if (__popc(cols) <= __popc(rows)) {
+      if (kma <= kDenseKma && min(__popc(cols), __popc(rows)) > kDense) {
+        // many are left: the rows are bounded against each block of eight starts by itself
+        float lo = col ? Pi.x : INFINITY, hi = col ? Pi.x : -INFINITY;
+        float c0 = col ? Pi.y : INFINITY, c1 = col ? Pi.y : -INFINITY;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+          lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+          hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+          c0 = fminf(c0, __shfl_xor_sync(0xffffffffu, c0, o));
+          c1 = fmaxf(c1, __shfl_xor_sync(0xffffffffu, c1, o));
+        }
+        for (int q = 0; q < 32; q += 8) {
+          unsigned part = cols & (0xffu << q);
+          if (!part) continue;
+          const float blo = __shfl_sync(0xffffffffu, lo, q), bhi = __shfl_sync(0xffffffffu, hi, q);
+          const float bc0 = __shfl_sync(0xffffffffu, c0, q), bc1 = __shfl_sync(0xffffffffu, c1, q);
+          const bool r = row && (unsigned)(e - (s32 + q) - kmi - 1) < (unsigned)(kma - kmi + 7) &&
+                         alive(fmaxf(Pe.x - blo, bhi - Pe.x), Pe.y - bc1, Pe.y - bc0, thr);
+          if (!__any_sync(0xffffffffu, r)) continue;
+          do {
+            const int b = __ffs(part) - 1;
+            part &= part - 1;
+            const float2 A = P[s32 + b];
+            if (r) consider(A, swz(s32 + b), Pe, e);
+          } while (part);
+        }
+      } else if (__popc(cols) <= __popc(rows)) {
         do {
           const int b = __ffs(cols) - 1;
           cols &= cols - 1;

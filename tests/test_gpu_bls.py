@@ -211,3 +211,28 @@ def test_kmi_past_the_range_of_widths(cuda, nb, kma):
     for kmi in (kma, 2 ** 31 - 1, -1, -100000, -2 ** 31):
         rec = api.refined_to_numpy(api.bls_refine(sr, p1, p2, X, T, off, nt, nb, kma, kmi, 5, 0.05, 0.02, K=8, S=4, M=4))
         assert not rec["sr"].any() and not rec["kk"].any()
+
+
+@pytest.mark.parametrize("nb,kma", [(100, 10), (100, 40), (256, 25), (300, 101), (512, 51), (512, 160), (512, 161), (1024, 102),
+                                    (1000, 33)])
+@pytest.mark.parametrize("kind", ["trend", "transit", "steps"])
+def test_units_with_many_windows_left(cuda, nb, kma, kind):
+    """Slow trends, deep transits and a flux of few values leave most windows of many units: the starts are then
+    bounded in blocks of eight up to the largest width that does so, all at once past it."""
+    n, nq, nf = 1200, 3, 12
+    rng = np.random.default_rng(nb + kma)
+    t = np.tile(((np.arange(n) + 0.3) * np.float32(0.0204)).astype(np.float32)[:, None], (1, nq))
+    x = rng.normal(0, 1e-3, (n, nq))
+    if kind == "trend":
+        x = 0.05 * x + np.sin(t / (2.0 + np.arange(nq)))
+    if kind == "transit":
+        x = x - 5e-2 * (np.mod(t + 0.1 * np.arange(nq), 3.3) < 0.25)
+    if kind == "steps":
+        x = np.round(x * 500) / 500
+    x = x.astype(np.float32)
+    off, ntrue = np.zeros(nq, np.float32), np.full(nq, n, np.uint32)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    sr, p1, p2 = api.geebls(d(x), d(t), d(off), d(ntrue.astype(np.int32)), nf, nb, kma, 1, 5, 0.05, 0.05)
+    osr, op1, op2, opmax = oracle.bls(x, t, nf, nb, kma, 1, 5, np.float32(0.05), np.float32(0.05), offset=off, ntrue=ntrue)
+    _check_spectrum(sr.cpu().numpy(), p1.cpu().numpy(), p2.cpu().numpy(), osr, op1, op2, opmax, x, t,
+                    dict(nb=nb, fmin=0.05, df=0.05), off, ntrue)
