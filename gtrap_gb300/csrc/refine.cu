@@ -249,7 +249,9 @@ __device__ __forceinline__ float ll_mag(long long v) {
 // finding peak and scale again, every window twice and 64-bit compare-and-swap atomics; 303 us with
 // those gone; 230 us with a shift for the fine bin where S is a power of two, windows screened
 // by a product and no quotient, and 12 warps a block for 8: 256 threads take 243 us, 512 (fewer
-// registers each) 275 us).
+// registers each) 275 us).  Where a block has under seven trials its warps share them as teams: a lone
+// curve of 9000 samples, nb = 2048, kma = 205 in 42-53 us a call (a warp a trial, the block's
+// others idle: 104 for one of 500 samples, 490 with 64 fine bins a bin; now 39 and 111).
 __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ long long shl[kThreads / 32];
@@ -344,7 +346,8 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
   stot = block_sum<long long>(stot, shl);
   __syncthreads();
 
-  // ---- a warp per trial from here on: exclusive prefix sums, then stage 1, every window of whole
+  // ---- a warp per trial, or a team of warps where the block has fewer trials than half its warps (a few
+  // curves, or neighbourhoods that leave room for little), from here on: exclusive prefix sums, then stage 1, every window of whole
   // bins in the neighbourhood (width in (kmi, kma] bins), then stage 2, fine edges within one bin of
   // the stage-1 window's edges (width in (kmi S, kma S] fine bins).  Both stages screen in FP32 with
   // error bounds: windows whose upper bound reaches a lower bound of the largest power are compared
@@ -357,12 +360,27 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
   auto warp_max = [](float v) {   // non-negative values
     return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
   };
-  for (uint32_t g = warp; g < nk; g += kThreads / 32) {
+  __shared__ float team_pm[kThreads / 32], team_thr[kThreads / 32], team_top[kThreads / 32];
+  __shared__ double best_p[kThreads / 32];
+  __shared__ uint32_t best_a[kThreads / 32], best_b[kThreads / 32];
+  const int W = max(1, kThreads / 32 / (int)nk), team = warp / W, member = warp - team * W;
+  auto team_sync = [&]() {
+    if (W == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(32 * W) : "memory");
+  };
+  auto team_max = [&](float v, float *sh) {   // of warp-uniform values
+    if (W == 1) return v;
+    if (lane == 0) sh[warp] = v;
+    team_sync();
+    for (int m = 0; m < W; ++m) v = fmaxf(v, sh[team * W + m]);
+    return v;
+  };
+  for (uint32_t g = team; g < nk; g += kThreads / 32 / W) {   // (a team: one trial)
     long long *H = hs + (size_t)g * E;
     int *C = hc + (size_t)g * E;
     float2 *P = cp + (size_t)g * (L + 1);
     float *R = rm + (size_t)g * (L + 1);
-    {
+    if (member == 0) {
       // each lane a run of entries (an odd number: fewer bank conflicts), a warp scan of the totals
       const uint32_t run = ((E + 31) / 32) | 1u;
       const uint32_t b0 = min(E, lane * run), b1 = min(E, b0 + run);
@@ -411,19 +429,19 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
         ec += vc;
       }
     }
-    __syncwarp();
+    team_sync();
     // the coarse entries as floats and their largest magnitude.  Quantised units: |H| < 2^63 whole numbers,
     // so a square stays below 2^126, and a power that is not zero above 2^-62: nothing leaves the normal
     // range (in real units the threshold of a long curve of 2^-50 flux is subnormal, and a bound
     // multiplied out of it passes over the best window)
     float pm = 0.0f;
-    for (int e = lane; e <= iL; e += 32) {
+    for (int e = 32 * member + lane; e <= iL; e += 32 * W) {
       const float v = __ll2float_rn(H[e * S]);
       P[e] = make_float2(v, (float)C[e * S]);
       pm = fmaxf(pm, fabsf(v));
     }
-    pm = warp_max(pm);
-    __syncwarp();
+    pm = team_max(warp_max(pm), team_pm);
+    __syncwarp();   // (a team's entries: its barrier)
     // |P - exact| <= 2^-24 |exact| per entry, so a difference is off by at most 2^-23 pmax
     // plus 2^-24 of itself (both taken twice here); den is exact to 2^-24 and the quotient
     // from __fdividef within 2 ulp, inside the 2^-20 factors
@@ -459,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
         if (ws >= 0 && we <= iL && we - ws > kmi && we - ws <= kma) thr = fmaxf(thr, lower(P[ws], P[we]));
       }
       thr = warp_max(thr);
-      for (int s = 0; s < iL; ++s) {
+      for (int s = member; s < iL; s += W) {
         const float2 A = P[s];
         const int wmax = min(kma, iL - s);
         bool hit = false;
@@ -477,20 +495,26 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
         if (any) thr = warp_max(thr);
         if (lane == 0) R[s] = any ? 1.0f : 0.0f;
       }
+      thr = team_max(thr, team_thr);
     }
-    __syncwarp();
+    __syncwarp();   // (a warp reads its own rows of R)
     double bp = -1.0;
     uint32_t ba = UINT_MAX, bb = UINT_MAX;
-    auto warp_best = [&]() {   // fixed-order argmax
+    auto trial_best = [&]() {   // fixed-order argmax
       for (int o = 16; o > 0; o >>= 1) {
         const double op = __shfl_xor_sync(0xffffffffu, bp, o);
         const uint32_t oa = __shfl_xor_sync(0xffffffffu, ba, o);
         const uint32_t ob = __shfl_xor_sync(0xffffffffu, bb, o);
         if (better(op, oa, ob, bp, ba, bb)) { bp = op; ba = oa; bb = ob; }
       }
+      if (W == 1) return;
+      if (lane == 0) { best_p[warp] = bp; best_a[warp] = ba; best_b[warp] = bb; }
+      team_sync();
+      for (int m = team * W; m < team * W + W; ++m)
+        if (better(best_p[m], best_a[m], best_b[m], bp, ba, bb)) { bp = best_p[m]; ba = best_a[m]; bb = best_b[m]; }
     };
     for (int s0 = 0; s0 < iL; s0 += 32) {
-      const bool in = s0 + lane < iL && R[s0 + lane] > 0.0f;
+      const bool in = s0 + lane < iL && (W == 1 || (s0 + lane) % W == member) && R[s0 + lane] > 0.0f;
       for (unsigned rows = __ballot_sync(0xffffffffu, in); rows; rows &= rows - 1) {
         const int s = s0 + __ffs(rows) - 1;
         const float2 A = P[s];
@@ -503,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
         }
       }
     }
-    warp_best();
+    trial_best();
     if (ba != UINT_MAX) {
       const uint32_t a0 = ba > S ? ba - S : 0u, a1 = ba + S < LS ? ba + S : LS;
       const uint32_t b0 = bb > S ? bb - S : 0u, b1 = bb + S < LS ? bb + S : LS;
@@ -517,18 +541,19 @@ __global__ void __launch_bounds__(kThreads, 2) refine_trial_kernel(const RefArgs
         return kk > kkmi_f && den > 0.0f ? __fdividef(sv * sv, den) : 0.0f;
       };
       float top = 0.0f;
-      for (uint32_t q = lane; q < na * nbw; q += 32) top = fmaxf(top, approx(a0 + q / nbw, b0 + q % nbw));
-      const float low = warp_max(top) * (1.0f - 1.0f / 262144.0f);
-      for (uint32_t q = lane; q < na * nbw; q += 32) {
+      const uint32_t q0 = 32 * member + lane, dq = 32 * W;
+      for (uint32_t q = q0; q < na * nbw; q += dq) top = fmaxf(top, approx(a0 + q / nbw, b0 + q % nbw));
+      const float low = team_max(warp_max(top), team_top) * (1.0f - 1.0f / 262144.0f);
+      for (uint32_t q = q0; q < na * nbw; q += dq) {
         const uint32_t ws = a0 + q / nbw, we = b0 + q % nbw;
         if (we <= ws || we - ws <= wmin || we - ws > wmax) continue;
         if (approx(ws, we) < low) continue;
         double pw;
         if (power((int)ws, (int)we, pw) && better(pw, ws, we, bp, ba, bb)) { bp = pw; ba = ws; bb = we; }
       }
-      warp_best();
+      trial_best();
     }
-    if (lane == 0) {
+    if (lane == 0 && member == 0) {
       Part &o = pt[g];
       o.pw = ba == UINT_MAX ? -1.0 : bp;
       o.s = ba == UINT_MAX ? 0 : H[bb] - H[ba];

@@ -278,3 +278,31 @@ def test_refine_scales_with_the_flux(cuda, exponent):
         np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
     for key in ("sr", "depth"):
         np.testing.assert_array_equal(got[key], np.ldexp(ref[key], exponent), err_msg=key)
+
+
+@pytest.mark.parametrize("K,S,M,kma", [(1, 8, 8, 103), (2, 64, 2, 60), (4, 3, 4, 26), (16, 16, 8, 200), (32, 1, 8, 205), (64, 8, 8, 400)])
+def test_refine_trials_by_warps_and_by_teams(cuda, K, S, M, kma):
+    """A block's trials take a warp each, or teams of two to twelve where there are few of them: one curve, a few and
+    many (one trial a block up to dozens) give the same bits, and the oracle's record."""
+    n, nb, nf = 2500, 2048, 60
+    rng = np.random.default_rng(K + kma)
+    t = (np.arange(n) * np.float32(0.0204)).astype(np.float32)
+    x = rng.normal(0, 1e-3, n).astype(np.float32) - np.float32(2e-3) * (np.mod(t - 0.7, 3.1) < 0.2).astype(np.float32)
+    g = dict(nf=nf, nb=nb, kma=kma, kmi=1, kkmi=8, fmin=0.2, df=0.01)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    T, X = d(t)[:, None], d(x)[:, None]
+    first = None
+    for count in (1, 2, 7, 40, 310):
+        args = (X.expand(n, count).contiguous(), T.expand(n, count).contiguous(), torch.zeros(count, device=cuda),
+                torch.full((count,), n, dtype=torch.int32, device=cuda))
+        if first is None:
+            sr, p1, p2 = api.geebls(*args, nf, nb, kma, 1, 8, 0.2, 0.01)
+        rep = lambda v: v.expand(count, nf).contiguous()
+        recs = api.refined_to_numpy(api.bls_refine(rep(sr), rep(p1), rep(p2), *args, nb, kma, 1, 8, 0.2, 0.01, K=K, S=S, M=M))
+        if first is None:
+            first = recs[0].tobytes()
+            host = [v.cpu().numpy()[0] for v in (sr, p1, p2)]
+            o = OR.refine_curve(t, x, 0.0, n, host[0], host[1].view(np.uint32), host[2].view(np.uint32), 0.2, 0.01, nb, kma,
+                                1, 8, K=K, S=S, M=M)
+            _check(recs[0], o)
+        assert all(r.tobytes() == first for r in recs), count
