@@ -90,3 +90,17 @@ def test_image_offsets_keep_the_order(cuda, n, nq):
     got = api.offset(torch.from_numpy(resid).to(cuda), torch.from_numpy(tu).to(cuda)).cpu().numpy()
     want = np.array([_offset_in_order(resid[:, q], tu[:, q]) for q in range(nq)], np.float32)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("nq", [600, 700, 1003])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 257, 4096, 4097])
+def test_offsets_of_many_short_curves_keep_the_order(cuda, n, nq):
+    """Many curves of up to 4096 samples take one block a group, longer or fewer ones a cluster: the same order."""
+    rng = np.random.default_rng(n + nq)
+    resid = rng.normal(1e-3, 1e-3, size=(n, nq)).astype(np.float32)
+    tu = np.tile(np.arange(n, dtype=np.float32)[:, None], (1, nq))
+    tu[rng.random((n, nq)) < 0.1] = -1000.0
+    resid[(tu < 0) & (rng.random((n, nq)) < 0.2)] = np.nan
+    got = api.offset(torch.from_numpy(resid).to(cuda), torch.from_numpy(tu).to(cuda)).cpu().numpy()
+    for q in (0, 1, 15, 16, 31, 300, nq - 2, nq - 1):
+        assert got[q] == _offset_in_order(resid[:, q], tu[:, q]), q
