@@ -715,7 +715,12 @@ int gtrap_peakstat(const float *sn, const uint64_t *off, const uint32_t *n, uint
   if (smem > gtrap_peakstat_max_samples())
     return fail(GTRAP_ERR_UNSUPPORTED, "peakstat: series of %u samples exceed the %zu that fit in shared memory",
                 max_n, gtrap_peakstat_max_samples());
-  if (smem <= staged_max()) {
+  // Short series with wide windows, many of them: the staged kernel's walks over a list that one window spans leave
+  // most of its 1024 threads idle, and it runs one block an SM.  Staged / the other, 5000 series: mpd 100, 200
+  // samples 1783 / 1216 us, 500 2297 / 1934, 700 2732 / 2783; mpd 17, 200 samples 1264 / 1189; 100 series
+  // of 200 with mpd 100 87 / 131; mpd 16, the masks' reach, 5000 of 200 891 / 1176.
+  const bool wide_short = mpd > 16 && smem <= 512 && ncurves > 4u * (uint32_t)sm_count();
+  if (smem <= staged_max() && !wide_short) {
     const size_t bytes = staged_bytes(smem);
     GTRAP_TRY(ensure_smem((const void *)peakstat_staged_kernel, bytes, "peakstat"));
     peakstat_staged_kernel<<<ncurves, kStThreads, bytes, stream>>>(sn, (const unsigned long long *)off, n, (size_t)stride,

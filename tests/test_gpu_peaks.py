@@ -149,3 +149,14 @@ def test_median_of_a_series_with_nan(cuda, bits, n, count, shift):
                                 torch.from_numpy(lens.astype(np.int32)).to(cuda), 1, int(lens.max()), 10, 4, 8)
         got = api.stats_to_numpy(st)[0]["median"]
         assert np.isnan(got) if np.isinf(ref) else got == ref, (len(xs), got, ref)
+
+
+@pytest.mark.parametrize("n,nq,mpd", [(512, 700, 17), (513, 700, 17), (200, 700, 100), (200, 600, 100), (40, 2000, 16), (40, 2000, 40)])
+def test_many_short_series_with_wide_windows(cuda, n, nq, mpd):
+    """At both ends of the rule that takes them to the kernel of the longest series."""
+    xs = [_series(3000 + q % 9, n) for q in range(9)]
+    img = np.stack([xs[q % 9] for q in range(nq)], axis=1)
+    st, idx, val = api.tls_peakstat(torch.from_numpy(img).to(cuda), mpd=mpd, ntop=3, k=6)
+    st, idx, val = api.stats_to_numpy(st), idx.cpu().numpy(), val.cpu().numpy()
+    for q in list(range(9)) + [nq - 1]:
+        _check(st[q], idx[q], val[q], img[:, q], mpd, 3, 6)
