@@ -236,3 +236,21 @@ def test_units_with_many_windows_left(cuda, nb, kma, kind):
     osr, op1, op2, opmax = oracle.bls(x, t, nf, nb, kma, 1, 5, np.float32(0.05), np.float32(0.05), offset=off, ntrue=ntrue)
     _check_spectrum(sr.cpu().numpy(), p1.cpu().numpy(), p2.cpu().numpy(), osr, op1, op2, opmax, x, t,
                     dict(nb=nb, fmin=0.05, df=0.05), off, ntrue)
+
+
+@pytest.mark.parametrize("n,nb,kma", [(300, 96, 95), (300, 256, 120), (3000, 1024, 500), (2000, 100, 45)])
+def test_windows_that_hold_every_sample(cuda, n, nb, kma):
+    """Fewer cycles than a window is wide: a window holds every sample, and where the flux does not sum to zero its
+    power is infinite, as in FP64; at the other frequencies the spectrum is finite."""
+    rng = np.random.default_rng(nb)
+    nq, nf = 2, 24
+    t = np.tile((np.arange(n) * np.float32(0.02)).astype(np.float32)[:, None], (1, nq))
+    x = (0.01 + rng.normal(0, 1e-3, (n, nq))).astype(np.float32)
+    off, ntrue = np.zeros(nq, np.float32), np.full(nq, n, np.uint32)
+    fmin = df = float(np.float32(0.06 / (n * 0.02)))     # 0.06, 0.12, ... 1.44 cycles
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    sr, p1, p2 = api.geebls(d(x), d(t), d(off), d(ntrue.astype(np.int32)), nf, nb, kma, 1, 5, fmin, df)
+    osr, op1, op2, opmax = oracle.bls(x, t, nf, nb, kma, 1, 5, np.float32(fmin), np.float32(df), offset=off, ntrue=ntrue)
+    assert np.isinf(osr).any() and np.isfinite(osr).any()
+    _check_spectrum(sr.cpu().numpy(), p1.cpu().numpy(), p2.cpu().numpy(), osr, op1, op2, opmax, x, t,
+                    dict(nb=nb, fmin=fmin, df=df), off, ntrue)

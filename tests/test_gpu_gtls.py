@@ -133,3 +133,30 @@ def test_gtls_half_tiles(cuda, nt, nw):
     for one, many in zip(run(1, nt), run(nq if nt == 1000 else 64 * nq, nt)):
         assert torch.equal(one[:, 0].view(torch.int32), many[:, 0].view(torch.int32))
         assert torch.equal(one[:, 0].view(torch.int32), many[:, -1].view(torch.int32))
+
+
+@pytest.mark.parametrize("bits", [0x7fc00000, 0xffc00000, 0x7fc0dead])
+def test_gtls_nan_flux_beside_masked_samples(cuda, bits):
+    """A sample that counts but has no flux (NaN, whatever its payload: masked samples carry one of their own) takes
+    the S/N of every epoch whose scoop holds it (the sums are differences of prefixes); no output is NaN, epochs
+    far from it keep their bits, and half tiles and whole tiles agree."""
+    n = 3000
+    rng = np.random.default_rng(21)
+    tu = ((np.arange(n) + 0.5) * synth.TESS_CADENCE).astype(np.float32)[:, None]
+    tu[1480:1500] = -1000.0                      # the only masked samples
+    lc = rng.normal(0, 1e-3, (n, 1)).astype(np.float32)
+    g = synth.tls_grid(nw=8, nl=6)
+    clean = _run(cuda, lc, tu, n, g)
+    bad = lc.copy()
+    bad.view(np.uint32)[1505, 0] = bits
+    bad.view(np.uint32)[1490, 0] = bits          # masked: not looked at
+    got = _run(cuda, bad, tu, n, g)
+    assert not any(np.isnan(a).any() for a in got)
+    near = np.abs(np.arange(n) - 1505) <= g["nsc"] // 2 - 1
+    assert (got[0][near] == 0).all() and (clean[0][near] > 0).any()
+    far = np.abs(np.arange(n) - 1505) > g["nsc"] + 64
+    for a, b in zip(got, clean):
+        np.testing.assert_array_equal(a[far], b[far])
+    wide = _run(cuda, np.repeat(bad, 120, 1), np.repeat(tu, 120, 1), n, g)
+    for a, b in zip(got, wide):
+        np.testing.assert_array_equal(a[:, 0], b[:, 7])
