@@ -1194,13 +1194,16 @@ constexpr uint32_t kFewF = 4;
 // frequencies: 4122 / 4174; the step to the next frequency is a product a sample), not for 4096 bins, whose steps
 // pass many such places (2 x 40,000, 400 frequencies: 132 / 188), and not for few bins, where some
 // frequencies are folded again in 64 bits, best several in a block at once (2 x 40,000, nb = 100: 715 / 865).
+// A launch of hundreds of waves waits for no block (128 curves of 65,536 and 16,384 frequencies, 1150 waves: 114.8 / 115.7 ms).
 constexpr uint32_t kSpreadMinN = 8192, kSpreadMinNb = 256, kSpreadMaxNb = 2048;
+constexpr uint64_t kSpreadWaves = 128;
 // the same for the segments of a work queue, by their number (their lengths are on the device): one curve of
 // 65,000 samples, 1800 frequencies, nb = 2048 417 / 268 us, twelve of 18,000, 2000 frequencies, nb = 512
 // 846 / 768; a batch of 80 curves of all lengths 10,150 / 10,212
 constexpr uint32_t kSpreadSegments = 16;
-bool spread_tiles(uint32_t n, uint32_t nb) {
-  return n >= kSpreadMinN && nb >= kSpreadMinNb && nb <= kSpreadMaxNb;
+bool spread_tiles(uint32_t n, uint32_t nb, uint64_t blocks) {
+  return n >= kSpreadMinN && nb >= kSpreadMinNb && nb <= kSpreadMaxNb &&
+         blocks <= kSpreadWaves * kMinBlocks * gtrap::sm_count();
 }
 
 int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const float *lc,
@@ -1279,7 +1282,7 @@ int run_bls(bool full, float *blsp, uint32_t *phase1, uint32_t *phase2, const fl
   if (blocks >= (1ull << 31)) return fail(GTRAP_ERR_INVALID_ARG, "%s: grid too large", name);
   const void *fn;
   const int mode = !exact ? 2 : (gtrap::is_pow2(nb) ? 0 : 1);
-  const bool spread = spread_tiles(n, nb);
+  const bool spread = spread_tiles(n, nb, blocks);
 #define GTRAP_BLS_LAUNCH(RR, MM)                                                          \
   fn = spread ? (const void *)bls_fold_scan_kernel<RR, MM, true>                           \
               : (const void *)bls_fold_scan_kernel<RR, MM, false>;                         \
