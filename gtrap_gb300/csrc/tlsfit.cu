@@ -11,8 +11,9 @@
 // over |t - t0| <= W/2 (divx), the region sums, and the residual with the fitted depth.  The
 // region masks, the boundary expressions (-W/4 - L/2 evaluated as (-W/4) - L/2 ...), the
 // nansum semantics (counts over all samples, sums over finite flux) and the formulas of denA,
-// numB, Hmax and the residual follow the reference term by term; only the summation order
-// differs (warp order instead of numpy's pairwise sums).
+// numB, Hmax and the residual follow the reference's.  Two things differ in rounding alone: a thread adds
+// its samples in time order (numpy adds pairwise), and takes each product into its sum by one FMA, so
+// that a term is rounded once and not twice.
 //
 // Bound by the FP64 pipe, which takes a warp's instruction 16 cycles here: a sample is tested for NaN
 // and infinity on its bits, and products go into their sums by one FMA (7 FP64 instructions a window
