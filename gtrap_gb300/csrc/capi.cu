@@ -115,7 +115,7 @@ int ensure_smem(const void *func, size_t bytes, const char *what) {
   if (bytes + static_bytes > (size_t)max_smem_optin())
     return fail(GTRAP_ERR_INVALID_ARG, "%s: needs %zu + %zu bytes of shared memory, device allows %d",
                 what, bytes, static_bytes, max_smem_optin());
-  if (bytes <= 48 * 1024) return GTRAP_OK;
+  if (bytes + static_bytes <= 48 * 1024) return GTRAP_OK;   // (static bytes count here too)
   // The attribute is per function and per device; setting it again is harmless, and
   // the call is cheap next to a launch, so it is simply repeated (also during capture).
   std::lock_guard<std::mutex> lock(g_attr_mutex);
