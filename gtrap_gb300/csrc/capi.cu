@@ -116,11 +116,13 @@ int ensure_smem(const void *func, size_t bytes, const char *what) {
     return fail(GTRAP_ERR_INVALID_ARG, "%s: needs %zu + %zu bytes of shared memory, device allows %d",
                 what, bytes, static_bytes, max_smem_optin());
   if (bytes + static_bytes <= 48 * 1024) return GTRAP_OK;   // (static bytes count here too)
-  // The attribute is per function and per device; setting it again is harmless, and
-  // the call is cheap next to a launch, so it is simply repeated (also during capture).
+  // The attribute is per function and per device, and a limit only: it is set to the most the function can
+  // have, whatever this launch needs, so that threads launching it at different sizes never lower it under one
+  // another.  Setting it again is harmless, and cheap next to a launch, so it is simply repeated (also during
+  // capture).
   std::lock_guard<std::mutex> lock(g_attr_mutex);
   cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)bytes);
+                                       max_smem_optin() - (int)static_bytes);
   if (e != cudaSuccess)
     return fail(GTRAP_ERR_CUDA, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
   return GTRAP_OK;

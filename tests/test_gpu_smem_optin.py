@@ -35,3 +35,37 @@ assert float(out[0].max()) > 0
 def test_first_launch_near_48_kb(cuda, code, n):
     res = subprocess.run([sys.executable, "-c", code.format(n=n)], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stderr[-800:]
+
+
+def test_threads_launching_one_kernel_at_different_sizes(cuda):
+    """Four threads, each on its own stream, with series of lengths of their own: no launch is refused for the size
+    that another thread has just asked for, and the results are those of each alone."""
+    import threading
+
+    import numpy as np
+    import torch
+    from gtrap_gb300 import api
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    errors = []
+
+    def work(n):
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                x = torch.from_numpy(np.abs(np.random.default_rng(n).normal(size=(n, 1))).astype(np.float32)).cuda()
+                ref = [v.clone() for v in api.tls_peakstat(x)[1:]]
+                for _ in range(1500):
+                    got = api.tls_peakstat(x)[1:]
+                assert all(torch.equal(a, b) for a, b in zip(ref, got))
+                s.synchronize()
+        except Exception as exc:   # (a thread's exception would not fail the test)
+            errors.append((n, exc))
+
+    try:
+        threads = [threading.Thread(target=work, args=(n,)) for n in (9000, 30000, 12000, 34000)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+    finally:
+        sys.setswitchinterval(interval)
+    assert not errors, errors[0]
