@@ -9,7 +9,8 @@ import pytest
 import torch
 
 import oracle
-from gtrap_gb300 import api, batch as B, synth
+from gtrap_gb300 import batch as B, synth
+from gtrap_gb300 import api
 
 pytestmark = pytest.mark.gpu
 
